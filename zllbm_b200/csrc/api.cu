@@ -41,6 +41,7 @@ struct Level {
     DeviceBuffer f;          // populations
     DeviceBuffer info;       // per-cell info (masked levels only)
     DeviceBuffer mrt64;      // dense M^-1 S M (FP64 storage)
+    std::vector<double> mrt64_host, mrt64_d_host;  // the FP64 matrices, passed to the step as kernel arguments
     DeviceBuffer feq_face;   // feq(rho0, U_face) per face, 6 * q doubles
     DeviceBuffer partial;    // conservation partial sums
     int partial_blocks = 0;
@@ -487,6 +488,8 @@ static int setup_level(zl_ctx* ctx, int level, const uint64_t* codes, int64_t n,
         }
     }
     p.omega32 = (float)(1. / p.tau);
+    p.inv_tau_hi = 1. / p.tau;
+    p.inv_tau_lo = std::fma(-p.inv_tau_hi, p.tau, 1.) / p.tau;
     for (int k = 0; k < q; ++k) {
         // fast-path MRT: shear moments relax with 1/tau through the SRT term; the others add
         // (s_k - 1/tau) / |M_k|^2 (conserved moments of neq vanish and stay out)
@@ -511,11 +514,15 @@ static int setup_level(zl_ctx* ctx, int level, const uint64_t* codes, int64_t n,
         if ((rc = alloc(ctx, L.mrt64, m.size() * sizeof(double)))) return rc;
         ZL_CUDA(ctx, cudaMemcpy(L.mrt64.ptr, m.data(), m.size() * sizeof(double), cudaMemcpyHostToDevice));
         p.mrt64 = (const double*)L.mrt64.ptr;
+        L.mrt64_host = m;
+        p.mrt64_host = L.mrt64_host.data();
         if (ctx->cfg.forcing) {
             host_mrt_matrix(dims, 1. / p.tau, true, m.data());
             if ((rc = alloc(ctx, L.mrt64_d, m.size() * sizeof(double)))) return rc;
             ZL_CUDA(ctx, cudaMemcpy(L.mrt64_d.ptr, m.data(), m.size() * sizeof(double), cudaMemcpyHostToDevice));
             p.mrt64_d = (const double*)L.mrt64_d.ptr;
+            L.mrt64_d_host = m;
+            p.mrt64_d_host = L.mrt64_d_host.data();
         }
     }
     if (ctx->cfg.forcing) {

@@ -4,6 +4,8 @@
 // step kernel variants in parallel translation units.  The launch sets of launch.cuh call them
 // through the declarations there.
 #pragma once
+#include <cstring>
+#include "f64_kernel.cuh"
 #include "launch.cuh"
 
 namespace zl {
@@ -13,14 +15,34 @@ namespace step_impl {
 // are numbered over each x-y plane (no warp holds the few nodes left at a row's end on its own),
 // rows' end nodes last when the x axis is bounded; a level of a few thousand nodes takes one-warp
 // blocks, so that its launch still reaches every SM.
-// (Measured: the flow past a cube 3 % faster; D2Q9 levels are faster per row, 3 % on the
-// cylinder flow.)
+// (Measured: the flow past a cube 3 % faster.)  D2Q9 levels take blocks of 32 x 4 nodes: 257^2 is 771
+// blocks of 128 along its rows, a wave and a bit of the FP64 step, and 585 of 32 x 4 (FP64, per step:
+// 257^2 5.0 -> 3.8 us, 385^2 6.5 -> 5.8, 1025^2 27.7 -> 26.0; numbering threads over the plane 4.1, 6.3, 25.6,
+// but 3.6 instead of 3.2 at 33^2).
+template <class S, class L, int C, bool O, bool B, bool M, int X>
+cudaError_t launch_one(S* f, const LevelGeom& geo, const StepParams& p, dim3 g, dim3 b, cudaStream_t s) {
+    // FP64 MRT with Smagorinsky keeps the general kernel, which builds the matrix node by node
+    if constexpr (sizeof(S) == 8 && !(C == kMrt && (X & kExtLes))) {
+        MrtArg<L::kQ, C == kMrt, (X & kExtForce) != 0> m;
+        if constexpr (C == kMrt) std::memcpy(m.a, p.mrt64_host, sizeof(m.a));
+        if constexpr (C == kMrt && (X & kExtForce)) std::memcpy(m.b, p.mrt64_d_host, sizeof(m.b));
+        ZL_LAUNCH_DEP(aa_step_f64_kernel<L, C, O, B, M, X>, g, b, 0, s, f, geo, p, m);
+    } else {
+        ZL_LAUNCH_DEP(aa_step_kernel<L, S, C, O, B, M, X>, g, b, 0, s, f, geo, p);
+    }
+    return cudaGetLastError();
+}
+
 template <class S, class L, int C, bool O, bool B, bool M, int X = 0>
 cudaError_t step_one(S* f, const LevelGeom& geo, const StepParams& p, cudaStream_t s) {
     dim3 g, b;
     step_shape(geo, L::kDims, g, b);
     const bool default_shape = geo.block[0] == 0 || geo.block[0] == kRowKernelBlockX;
     const long long plane = (long long)geo.n[0] * geo.n[1];
+    if (L::kDims == 2 && default_shape) {
+        b = dim3(32, 4);
+        g = dim3((geo.n[0] + 31) / 32, (geo.n[1] + 3) / 4);
+    }
     if (L::kDims == 3 && default_shape && (geo.n[0] & 31) && plane < (1ll << 31)) {
         LevelGeom fg = geo;
         // a non-periodic x axis: every row's two end nodes patch missing upstream values, and
@@ -30,12 +52,9 @@ cudaError_t step_one(S* f, const LevelGeom& geo, const StepParams& p, cudaStream
         fg.flat = ends_last ? 2 : 1;
         fg.fn0 = FastDiv::make((uint32_t)(ends_last ? geo.n[0] - 2 : geo.n[0]));
         const unsigned bs = plane * g.z >= 148ll * 128 * 8 ? 128u : 32u;
-        ZL_LAUNCH_DEP(aa_step_kernel<L, S, C, O, B, M, X>, dim3((unsigned)((plane + bs - 1) / bs), 1, g.z), dim3(bs), 0, s,
-                      f, fg, p);
-        return cudaGetLastError();
+        return launch_one<S, L, C, O, B, M, X>(f, fg, p, dim3((unsigned)((plane + bs - 1) / bs), 1, g.z), dim3(bs), s);
     }
-    ZL_LAUNCH_DEP(aa_step_kernel<L, S, C, O, B, M, X>, g, b, 0, s, f, geo, p);
-    return cudaGetLastError();
+    return launch_one<S, L, C, O, B, M, X>(f, geo, p, g, b, s);
 }
 
 template <class S, int C, bool O>
