@@ -223,8 +223,8 @@ int zl_set_batching(zl_ctx* ctx, int enabled);
    amr_project/grid/grid_manager.cpp:997-1023). */
 int zl_set_level_streams(zl_ctx* ctx, int enabled);
 
-/* Replay zl_advance as a captured CUDA graph of two background steps (every launch of the
-   sub-cycled order, transfers and boundary passes included).  The graph is re-captured after any
+/* Replay zl_advance as a captured CUDA graph of an even number of background steps (every launch
+   of the sub-cycled order, transfers and boundary passes included).  The graph is re-captured after any
    change of levels, interfaces, vertices or tuning.  Off by default. */
 int zl_set_graph(zl_ctx* ctx, int enabled);
 
