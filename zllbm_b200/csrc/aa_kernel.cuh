@@ -22,7 +22,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <cstdint>
-#include "level_params.cuh"
+#include "fused_collide.cuh"
 #include "pdl.cuh"
 
 namespace zl {
@@ -799,7 +799,10 @@ __device__ __forceinline__ void moment_apply(const float* x, const float* coef, 
     }
 }
 
-template <class L, bool Les>
+// Explicit (FP32 storage): the D3Q19 collisions of fused_collide.cuh, whose bits do not depend on how
+// many nodes a thread updates; the 16-bit storages keep the forms above, which their one-node kernel
+// has always rounded with (their pair and row kernels differ from it in rounding).
+template <class L, bool Les, bool Explicit>
 __device__ __forceinline__ void collide_dev(const float* d, float* out, const StepParams& p, int coll, float* mac,
                                             const NodeForce* nf, float les_c = 0.f) {
     using Tb = Tables<L>;
@@ -807,7 +810,23 @@ __device__ __forceinline__ void collide_dev(const float* d, float* out, const St
     // a node whose force is exactly zero (every node of a forced level outside the immersed-
     // boundary band, with no constant force) takes the unforced update: the Guo terms vanish
     if (nf && nf->F[0] == 0. && nf->F[1] == 0. && nf->F[2] == 0.) nf = nullptr;
-    if constexpr (L::kQ == 19) {
+    if constexpr (L::kQ == 19 && Explicit) {
+        const F1* d1 = reinterpret_cast<const F1*>(d);
+        F1 *o1 = reinterpret_cast<F1*>(out), *m1 = reinterpret_cast<F1*>(mac);
+        if (coll == kMrt && !nf) {
+            fused_collide<true, Les, false>(d1, o1, p, F1{les_c}, (const F1*)nullptr, m1);
+            return;
+        }
+        if (coll == kSrt) {
+            if (nf) {
+                const F1 F[3] = {{(float)nf->F[0]}, {(float)nf->F[1]}, {(float)nf->F[2]}};
+                fused_collide<false, Les, true>(d1, o1, p, F1{les_c}, F, m1);
+            } else {
+                fused_collide<false, Les, false>(d1, o1, p, F1{les_c}, (const F1*)nullptr, m1);
+            }
+            return;
+        }
+    } else if constexpr (L::kQ == 19) {
         if (coll == kMrt && !nf && !Les) {
             mrt_d3q19_fused(d, out, p, mac);
             return;
@@ -1029,7 +1048,7 @@ __device__ __forceinline__ void aa_node(S* __restrict__ f, const LevelGeom& geo,
         if constexpr (St::kDeviation) {
             // Smagorinsky constant C: the level's, or 18 c of the learned closure's last evaluation
             const float les_c = Les ? (p.c_node ? 18.f * __ldg(p.c_node + self) : (float)p.les_c) : 0.f;
-            collide_dev<L, Les>(pre, post, p, Coll, mac, Forced ? &nf : nullptr, les_c);
+            collide_dev<L, Les, sizeof(S) == 4>(pre, post, p, Coll, mac, Forced ? &nf : nullptr, les_c);
         } else {
             collide_exact<L, Les>(pre, post, p, Coll, mac, Forced ? &nf : nullptr);
         }
@@ -1147,7 +1166,7 @@ __device__ __forceinline__ void aa_node_periodic(S* __restrict__ f, const LevelG
     }
     if constexpr (St::kDeviation) {
         const float les_c = Les ? (p.c_node ? 18.f * __ldg(p.c_node + row + x) : (float)p.les_c) : 0.f;
-        collide_dev<L, Les>(pre, post, p, Coll, mac, Forced ? &nf : nullptr, les_c);
+        collide_dev<L, Les, sizeof(S) == 4>(pre, post, p, Coll, mac, Forced ? &nf : nullptr, les_c);
     } else {
         collide_exact<L, Les>(pre, post, p, Coll, mac, Forced ? &nf : nullptr);
     }

@@ -450,6 +450,7 @@ static int setup_level(zl_ctx* ctx, int level, const uint64_t* codes, int64_t n,
         ZL_CUDA(ctx, cudaGetLastError());
     }
     L.nodes = (long long)present;
+    geo.full = (long long)present == box_nodes;
     L.bnd = false;
     for (int a = 0; a < dims; ++a)
         if (!geo.periodic[a]) L.bnd = true;

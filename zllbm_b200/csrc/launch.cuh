@@ -70,6 +70,26 @@ inline bool pair_eligible(int dims, bool bnd, bool masked, const StepParams& p, 
     return dims == 3 && (geo.ring || (!bnd && !masked)) && !p.forced && !p.les && elem_bytes < 8;
 }
 
+// Full periodic D3Q19 boxes in FP32 take the two-nodes-per-thread kernel without being asked to, from
+// a size at which its fewer, heavier threads still fill the GPU: with the default block shape, and with
+// Smagorinsky whatever the (positive) shape, which then shapes the pair kernel's blocks.  Its results
+// have the one-node kernel's bits (fused_collide.cuh).  The 16-bit storages keep the kernel that their
+// rounding streams are numbered for.  p.macro: the transfer sources' macros are saved by the masked
+// one-node kernel only.
+// Measured us per step, one node / two nodes per thread:
+//                   80^3          96^3          112^3         128^3         256^3
+//   SRT          11.3 / 13.3   16.4 / 18.0   36.3 / 37.5   54.2 / 52.8   403 / 384
+//   MRT          12.3 / 14.3   19.5 / 19.0   40.0 / 39.0   58.4 / 53.6   435 / 385
+//   SRT + LES    14.4 / 15.5   22.9 / 20.7   47.0 / 40.0   67.7 / 53.7   508 / 389
+//   MRT + LES    18.9 / 18.1   30.6 / 24.1   55.0 / 42.2   77.9 / 55.6   581 / 407
+constexpr long long kPairMinNodes = 3ll << 19, kPairMinNodesLes = 1ll << 19;
+inline bool pair_default(int dims, const StepParams& p, int elem_bytes, const LevelGeom& geo) {
+    return dims == 3 && elem_bytes == 4 && geo.full && geo.periodic[0] && geo.periodic[1] && geo.periodic[2] &&
+           !p.forced && !p.macro && !(geo.n[0] & 1) && !(geo.stride & 1) &&
+           (p.les ? geo.block[0] >= 0 : geo.block[0] == 0) &&
+           (long long)geo.n[0] * geo.n[1] * geo.n[2] >= (p.les ? kPairMinNodesLes : kPairMinNodes);
+}
+
 // The one-warp-per-row kernel (row_kernel.cuh): full periodic D3Q19 boxes in 16-bit storage
 // with rows of 128 or 256 nodes, no forcing or LES.
 inline bool row_eligible(int dims, bool bnd, bool masked, const StepParams& p, int elem_bytes,

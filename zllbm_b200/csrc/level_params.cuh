@@ -53,6 +53,7 @@ struct LevelGeom {
     // sharded lattice): every upstream node is present, the z ones in the ghost planes, so the
     // kernels of full periodic boxes apply with z addressed through the ghost frame
     int ring;
+    int full;  // every cell of the box holds a node (also where info is kept for forcing or Smagorinsky)
     FastDiv fa0, fa1;  // division by a[0] and a[1] (cell index -> box coordinates)
     // D3Q19 step launches: planes [z0, z0 + zn) of the last axis; zn = 0: every plane
     int z0, zn;

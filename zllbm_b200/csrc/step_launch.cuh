@@ -57,7 +57,8 @@ cudaError_t step_one(S* f, const LevelGeom& geo, const StepParams& p, cudaStream
     return launch_one<S, L, C, O, B, M, X>(f, geo, p, g, b, s);
 }
 
-template <class S, int C, bool O>
+// Two nodes per thread; Les: Smagorinsky.  The default shape is 128 threads, as few rows as they cover.
+template <class S, int C, bool O, bool Les>
 cudaError_t step_pair(S* f, const LevelGeom& geo, const StepParams& p, cudaStream_t s) {
     if constexpr (Storage<S>::kDeviation) {
         if ((geo.n[0] & 1) || (geo.stride & 1)) {
@@ -66,9 +67,18 @@ cudaError_t step_pair(S* f, const LevelGeom& geo, const StepParams& p, cudaStrea
             g1.block[0] = g1.block[1] = 0;
             return step_one<S, D3Q19, C, O, false, false>(f, g1, p, s);
         }
+        LevelGeom pg = geo;
+        if (geo.block[0] == 0) {
+            int bx = 128;
+            while (bx > 32 && bx >= geo.n[0]) bx /= 2;  // n0 / 2 pairs in a row
+            pg.block[0] = -bx;
+            pg.block[1] = 128 / bx;
+        } else if (geo.block[0] > 0) {
+            pg.block[0] = -geo.block[0];
+        }
         dim3 g, b;
-        step_shape(geo, 3, g, b);
-        ZL_LAUNCH_DEP(aa_pair_kernel<S, C, O>, g, b, 0, s, f, geo, p);
+        step_shape(pg, 3, g, b);
+        ZL_LAUNCH_DEP(aa_pair_kernel<S, C, O, Les>, g, b, 0, s, f, geo, p);
         return cudaGetLastError();
     }
     return cudaErrorInvalidValue;
@@ -97,7 +107,11 @@ cudaError_t step_lco(bool bnd, bool masked, S* f, const LevelGeom& geo, const St
         if (geo.block[0] == kRowKernelBlockX && row_eligible(3, bnd, masked, p, (int)sizeof(S), geo))
             return step_row<S, C, O>(f, geo, p, s);
         if (geo.block[0] < 0 && pair_eligible(3, bnd, masked, p, (int)sizeof(S), geo))
-            return step_pair<S, C, O>(f, geo, p, s);
+            return step_pair<S, C, O, false>(f, geo, p, s);
+        if constexpr (sizeof(S) == 4) {
+            if (pair_default(3, p, (int)sizeof(S), geo))
+                return p.les ? step_pair<S, C, O, true>(f, geo, p, s) : step_pair<S, C, O, false>(f, geo, p, s);
+        }
     }
     if (p.forced || p.les) {
         if (!masked) return cudaErrorInvalidValue;
