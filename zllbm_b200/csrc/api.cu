@@ -1972,7 +1972,7 @@ int zl_ib_get_forces(zl_ctx* ctx, int level, double* vertex_forces, double* tota
         IbVertices v = ib_view(ctx, L, level);
         const double dx0 = ctx->cfg.dx > 0. ? ctx->cfg.dx : 1.;
         const double scale = ctx->dims == 3 ? 1. / dx0 / dx0 : 1. / dx0;
-        ib_total_kernel<<<1, 32, 0, ctx->stream>>>(v, scale, (double*)L.ib_total.ptr);
+        ib_total_kernel<<<1, kIbTotalThreads, 0, ctx->stream>>>(v, scale, (double*)L.ib_total.ptr);
         ZL_CUDA(ctx, cudaGetLastError());
         ZL_CUDA(ctx, cudaMemcpyAsync(total, L.ib_total.ptr, 3 * 8, cudaMemcpyDeviceToHost, ctx->stream));
     }

@@ -351,22 +351,42 @@ __global__ void __launch_bounds__(128) mlp_forward_kernel(const float* __restric
 }
 
 // ---------------------------------------------------------------- full-box I/O, features, filter
-__device__ __forceinline__ Coord box_coord(const LevelGeom& geo, long long i) {
+// Node i of the box (x fastest; a box holds fewer than 2^31 cells): multiply-shift divisions by n0 and n1.
+struct BoxDiv {
+    FastDiv n0, n1;
+};
+__device__ __forceinline__ Coord box_coord(const LevelGeom& geo, const BoxDiv& dv, uint32_t i) {
+    const uint32_t r = dv.n0.div(i), z = dv.n1.div(r);
     Coord c;
-    c.x[0] = (int)(i % geo.n[0]);
-    const long long r = i / geo.n[0];
-    c.x[1] = (int)(r % geo.n[1]);
-    c.x[2] = (int)(r / geo.n[1]);
+    c.x[0] = (int)(i - r * (uint32_t)geo.n[0]);
+    c.x[1] = (int)(r - z * (uint32_t)geo.n[1]);
+    c.x[2] = (int)z;
     return c;
 }
 
+// Slots of a node's post-stream populations in the given layout (post_stream_slot): the neighbours' rows
+// are formed once per node, not once per population.
+struct StreamSlots {
+    NodeCells<D3Q19> cell;
+    int self;
+    long long stride;
+    int even;
+    __device__ __forceinline__ StreamSlots(const LevelGeom& geo, const Coord& c, int even_layout)
+        : cell(geo, c), self(cell(0, 0, 0)), stride(geo.stride), even(even_layout) {}
+    __device__ __forceinline__ long long operator()(int q) const {
+        using Tb = Tables<D3Q19>;
+        if (even && q != 0) return Tb::opp(q) * stride + cell(-Tb::cx(q), -Tb::cy(q), -Tb::cz(q));
+        return q * stride + self;
+    }
+};
+
 template <class S>
-__global__ void set_equilibrium_kernel(S* __restrict__ f, LevelGeom geo, StepParams p, int even,
+__global__ void set_equilibrium_kernel(S* __restrict__ f, LevelGeom geo, StepParams p, int even, BoxDiv dv,
                                        const float* __restrict__ rho, const float* __restrict__ u, long long nn) {
     using Tb = Tables<D3Q19>;
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= nn) return;
-    const Coord c = box_coord(geo, i);
+    const StreamSlots slot(geo, box_coord(geo, dv, (uint32_t)i), even);
     const float r = rho[i], ux = u[i * 3], uy = u[i * 3 + 1], uz = u[i * 3 + 2];
     const float usq15 = 1.5f * (ux * ux + uy * uy + uz * uz);
 #pragma unroll
@@ -375,72 +395,116 @@ __global__ void set_equilibrium_kernel(S* __restrict__ f, LevelGeom geo, StepPar
         const float w = (float)Tb::w(q);
         // feq - w = w (rho - 1) + w rho (3 cu + 4.5 cu^2 - 1.5 u^2)
         const float d = w * fmaf(r, fmaf(cu, fmaf(4.5f, cu, 3.f), -usq15), r - 1.f);
-        Storage<S>::store(f + post_stream_slot<D3Q19>(geo, c, q, even), d, p);
+        Storage<S>::store(f + slot(q), d, p);
     }
 }
 
 template <class S>
-__device__ __forceinline__ void load_node(const S* f, const LevelGeom& geo, const Coord& c, int even, float* d) {
+__device__ __forceinline__ void load_node(const S* f, const StreamSlots& slot, float* d) {
 #pragma unroll
-    for (int q = 0; q < 19; ++q) d[q] = Storage<S>::load_raw(f + post_stream_slot<D3Q19>(geo, c, q, even));
+    for (int q = 0; q < 19; ++q) d[q] = Storage<S>::load_raw(f + slot(q));
 }
 
+constexpr int kMacroThreads = 256;
+
+// A block's velocities through shared memory, so that the (x, y, z) records leave as whole lines.
+__device__ __forceinline__ void store_velocities(float* __restrict__ u, long long base, long long nn, const float* v) {
+    __shared__ float rec[3 * kMacroThreads];
+    const int t = threadIdx.x;
+    rec[3 * t] = v[0];
+    rec[3 * t + 1] = v[1];
+    rec[3 * t + 2] = v[2];
+    __syncthreads();
+    const long long first = 3 * base, last = 3 * (nn - base < kMacroThreads ? nn : base + kMacroThreads);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const long long j = first + t + k * kMacroThreads;
+        if (j < last) u[j] = rec[t + k * kMacroThreads];
+    }
+}
+
+// rho and u of every node (Q populations in, 16 bytes out).  256^3 with 64-bit divisions, slot arithmetic per
+// population and velocities stored with stride three: FP32 520 us, FP16 947, FP64 599; now 312 (1.55 GB, 5.0
+// TB/s), 329 and 402.
 template <class S>
-__global__ void get_macros_kernel(const S* __restrict__ f, LevelGeom geo, StepParams p, int even,
-                                  float* __restrict__ rho, float* __restrict__ u, long long nn) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= nn) return;
-    float d[19], neq[19], mac[4];
-    load_node(f, geo, box_coord(geo, i), even, d);
-    feq_neq_dev<D3Q19>(d, neq, p.scale, p.inv_scale, mac);
-    rho[i] = mac[0];
-    u[i * 3] = mac[1];
-    u[i * 3 + 1] = mac[2];
-    u[i * 3 + 2] = mac[3];
+__global__ void __launch_bounds__(kMacroThreads) get_macros_kernel(const S* __restrict__ f, LevelGeom geo, StepParams p,
+                                                                   int even, BoxDiv dv, float* __restrict__ rho,
+                                                                   float* __restrict__ u, long long nn) {
+    const long long base = blockIdx.x * (long long)kMacroThreads, i = base + threadIdx.x;
+    float mac[4] = {0.f, 0.f, 0.f, 0.f};
+    if (i < nn) {
+        float d[19], neq[19];
+        load_node(f, StreamSlots(geo, box_coord(geo, dv, (uint32_t)i), even), d);
+        feq_neq_dev<D3Q19>(d, neq, p.scale, p.inv_scale, mac);
+        rho[i] = mac[0];
+    }
+    store_velocities(u, base, nn, mac + 1);
 }
 
 // FP64 storage (absolute populations): feq in the reference's arithmetic order from the FP32
 // fields, and rho / u by the reference's macro rule, rounded to FP32 on output.
-__global__ void set_equilibrium_f64_kernel(double* __restrict__ f, LevelGeom geo, int even,
+__global__ void set_equilibrium_f64_kernel(double* __restrict__ f, LevelGeom geo, int even, BoxDiv dv,
                                            const float* __restrict__ rho, const float* __restrict__ u, long long nn) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= nn) return;
-    const Coord c = box_coord(geo, i);
+    const StreamSlots slot(geo, box_coord(geo, dv, (uint32_t)i), even);
     double feq[19];
     feq_exact<D3Q19>((double)rho[i], (double)u[i * 3], (double)u[i * 3 + 1], (double)u[i * 3 + 2], feq);
 #pragma unroll
-    for (int q = 0; q < 19; ++q) f[post_stream_slot<D3Q19>(geo, c, q, even)] = feq[q];
+    for (int q = 0; q < 19; ++q) f[slot(q)] = feq[q];
 }
 
-__global__ void get_macros_f64_kernel(const double* __restrict__ f, LevelGeom geo, int even,
-                                      float* __restrict__ rho, float* __restrict__ u, long long nn) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= nn) return;
-    const Coord c = box_coord(geo, i);
-    double v[19], r, ux, uy, uz;
+__global__ void __launch_bounds__(kMacroThreads) get_macros_f64_kernel(const double* __restrict__ f, LevelGeom geo,
+                                                                       int even, BoxDiv dv, float* __restrict__ rho,
+                                                                       float* __restrict__ u, long long nn) {
+    const long long base = blockIdx.x * (long long)kMacroThreads, i = base + threadIdx.x;
+    float w[3] = {0.f, 0.f, 0.f};
+    if (i < nn) {
+        const StreamSlots slot(geo, box_coord(geo, dv, (uint32_t)i), even);
+        double v[19], r, ux, uy, uz;
 #pragma unroll
-    for (int q = 0; q < 19; ++q) v[q] = f[post_stream_slot<D3Q19>(geo, c, q, even)];
-    macro_exact<D3Q19>(v, r, ux, uy, uz);
-    rho[i] = (float)r;
-    u[i * 3] = (float)ux;
-    u[i * 3 + 1] = (float)uy;
-    u[i * 3 + 2] = (float)uz;
+        for (int q = 0; q < 19; ++q) v[q] = f[slot(q)];
+        macro_exact<D3Q19>(v, r, ux, uy, uz);
+        rho[i] = (float)r;
+        w[0] = (float)ux;
+        w[1] = (float)uy;
+        w[2] = (float)uz;
+    }
+    store_velocities(u, base, nn, w);
 }
 
 template <class S>
-__global__ void features_kernel(const S* __restrict__ f, LevelGeom geo, StepParams p, int even,
+__global__ void features_kernel(const S* __restrict__ f, LevelGeom geo, StepParams p, int even, BoxDiv dv,
                                 float* __restrict__ x, long long nn) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= nn) return;
     float d[19], neq[19], mac[4], v[kIn];
-    load_node(f, geo, box_coord(geo, i), even, d);
+    load_node(f, StreamSlots(geo, box_coord(geo, dv, (uint32_t)i), even), d);
     feq_neq_dev<D3Q19>(d, neq, p.scale, p.inv_scale, mac);
     features(mac[0], neq, (float)p.tau, v, nullptr, p.inv_scale);
 #pragma unroll
     for (int k = 0; k < kIn; ++k) x[i * kIn + k] = v[k];
 }
 
-// One thread per factor^3 block of nodes: block means of rho, u, u_a u_b and f - feq.
+// Adds one node's share of the filter: rho, u, u_a u_b and f - feq.
+__device__ __forceinline__ void filter_add(const float* d, const StepParams& p, float* acc) {
+    float neq[19], mac[4];
+    feq_neq_dev<D3Q19>(d, neq, p.scale, p.inv_scale, mac);
+    acc[0] += mac[0];
+    acc[1] += mac[1];
+    acc[2] += mac[2];
+    acc[3] += mac[3];
+    acc[4] += mac[1] * mac[1];
+    acc[5] += mac[2] * mac[2];
+    acc[6] += mac[3] * mac[3];
+    acc[7] += mac[1] * mac[2];
+    acc[8] += mac[1] * mac[3];
+    acc[9] += mac[2] * mac[3];
+#pragma unroll
+    for (int q = 0; q < 19; ++q) acc[10 + q] += neq[q] * p.inv_scale;
+}
+
+// Block means over factor^3 nodes, any factor: one thread per block.
 template <class S>
 __global__ void filter_kernel(const S* __restrict__ f, LevelGeom geo, StepParams p, int even, int factor, int ncx,
                               int ncy, int ncz, float* __restrict__ out) {
@@ -458,25 +522,54 @@ __global__ void filter_kernel(const S* __restrict__ f, LevelGeom geo, StepParams
                 c.x[0] = X * factor + dx;
                 c.x[1] = Y * factor + dy;
                 c.x[2] = Z * factor + dz;
-                float d[19], neq[19], mac[4];
-                load_node(f, geo, c, even, d);
-                feq_neq_dev<D3Q19>(d, neq, p.scale, p.inv_scale, mac);
-                acc[0] += mac[0];
-                acc[1] += mac[1];
-                acc[2] += mac[2];
-                acc[3] += mac[3];
-                acc[4] += mac[1] * mac[1];
-                acc[5] += mac[2] * mac[2];
-                acc[6] += mac[3] * mac[3];
-                acc[7] += mac[1] * mac[2];
-                acc[8] += mac[1] * mac[3];
-                acc[9] += mac[2] * mac[3];
-#pragma unroll
-                for (int q = 0; q < 19; ++q) acc[10 + q] += neq[q] * p.inv_scale;
+                float d[19];
+                load_node(f, StreamSlots(geo, c, even), d);
+                filter_add(d, p, acc);
             }
     const float inv = 1.f / (float)(factor * factor * factor);
 #pragma unroll
     for (int k = 0; k < 29; ++k) out[i * 29 + k] = acc[k] * inv;
+}
+
+// The same for factors that divide a warp: a warp takes 32 consecutive nodes of a row of the fine level
+// (coalesced loads; one thread per block strode by the factor), a thread sums the factor^2 nodes of its
+// column in the block, and a butterfly over the factor lanes of a block adds the columns.  The block's
+// lanes share its 29 stores.  256^3 by 4, FP32 (1.4 GB): 585 us with one thread per
+// block, 349 now.
+constexpr int kFilterThreads = 128;
+template <class S>
+__global__ void __launch_bounds__(kFilterThreads) filter_warp_kernel(const S* __restrict__ f, LevelGeom geo, StepParams p,
+                                                                     int even, int factor, int ncx, int ncy,
+                                                                     unsigned segments, float* __restrict__ out) {
+    const unsigned lane = threadIdx.x & 31u, seg = blockIdx.x * (kFilterThreads / 32) + (threadIdx.x >> 5);
+    if (seg >= segments) return;  // whole warps
+    const int x = (int)(seg * 32u + lane);
+    const bool live = x < geo.n[0];  // the factor divides n0: a block's lanes are all live or all not
+    float acc[29];
+#pragma unroll
+    for (int k = 0; k < 29; ++k) acc[k] = 0.f;
+    if (live) {
+        for (int dz = 0; dz < factor; ++dz)
+            for (int dy = 0; dy < factor; ++dy) {
+                Coord c;
+                c.x[0] = x;
+                c.x[1] = (int)blockIdx.y * factor + dy;
+                c.x[2] = (int)blockIdx.z * factor + dz;
+                float d[19];
+                load_node(f, StreamSlots(geo, c, even), d);
+                filter_add(d, p, acc);
+            }
+    }
+    const float inv = 1.f / (float)(factor * factor * factor);
+    for (int o = 1; o < factor; o <<= 1)
+#pragma unroll
+        for (int k = 0; k < 29; ++k) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+    if (!live) return;
+    const long long i = x / factor + (long long)ncx * (blockIdx.y + (long long)ncy * blockIdx.z);
+    const int sub = (int)lane & (factor - 1);
+#pragma unroll
+    for (int k = 0; k < 29; ++k)
+        if ((k & (factor - 1)) == sub) out[i * 29 + k] = acc[k] * inv;
 }
 
 // ---------------------------------------------------------------- training pairs
@@ -715,20 +808,27 @@ static cudaError_t dispatch_box(int op, void* f, const LevelGeom& geo, const Ste
                                 float* b, float* c, int factor, const int* nc, cudaStream_t s) {
     const long long nn = (long long)geo.n[0] * geo.n[1] * geo.n[2];
     const unsigned blocks = (unsigned)((nn + 255) / 256);
+    const BoxDiv dv{FastDiv::make((uint32_t)geo.n[0]), FastDiv::make((uint32_t)geo.n[1])};
     switch (op) {
         case kBoxSetEq:
-            set_equilibrium_kernel<S><<<blocks, 256, 0, s>>>((S*)f, geo, p, even, a, b, nn);
+            set_equilibrium_kernel<S><<<blocks, 256, 0, s>>>((S*)f, geo, p, even, dv, a, b, nn);
             break;
         case kBoxGetMacros:
-            get_macros_kernel<S><<<blocks, 256, 0, s>>>((const S*)f, geo, p, even, b, c, nn);
+            get_macros_kernel<S><<<blocks, kMacroThreads, 0, s>>>((const S*)f, geo, p, even, dv, b, c, nn);
             break;
         case kBoxFeatures:
-            features_kernel<S><<<blocks, 256, 0, s>>>((const S*)f, geo, p, even, b, nn);
+            features_kernel<S><<<blocks, 256, 0, s>>>((const S*)f, geo, p, even, dv, b, nn);
             break;
         case kBoxFilter: {
             const long long ncn = (long long)nc[0] * nc[1] * nc[2];
-            filter_kernel<S><<<(unsigned)((ncn + 127) / 128), 128, 0, s>>>((const S*)f, geo, p, even, factor, nc[0],
-                                                                            nc[1], nc[2], b);
+            if (factor <= 32 && !(factor & (factor - 1)) && nc[1] <= 65535 && nc[2] <= 65535) {
+                const unsigned segments = (unsigned)((geo.n[0] + 31) / 32), per = kFilterThreads / 32;
+                filter_warp_kernel<S><<<dim3((segments + per - 1) / per, nc[1], nc[2]), kFilterThreads, 0, s>>>(
+                    (const S*)f, geo, p, even, factor, nc[0], nc[1], segments, b);
+            } else {
+                filter_kernel<S><<<(unsigned)((ncn + 127) / 128), 128, 0, s>>>((const S*)f, geo, p, even, factor, nc[0],
+                                                                                nc[1], nc[2], b);
+            }
             break;
         }
         default:
@@ -761,10 +861,11 @@ cudaError_t closure_box_op(int op, int storage, void* f, const LevelGeom& geo, c
         case ZL_STORAGE_F64: {
             const long long nn = (long long)geo.n[0] * geo.n[1] * geo.n[2];
             const unsigned blocks = (unsigned)((nn + 255) / 256);
+            const BoxDiv dv{FastDiv::make((uint32_t)geo.n[0]), FastDiv::make((uint32_t)geo.n[1])};
             if (op == kBoxSetEq)
-                set_equilibrium_f64_kernel<<<blocks, 256, 0, s>>>((double*)f, geo, even, a, b, nn);
+                set_equilibrium_f64_kernel<<<blocks, 256, 0, s>>>((double*)f, geo, even, dv, a, b, nn);
             else if (op == kBoxGetMacros)
-                get_macros_f64_kernel<<<blocks, 256, 0, s>>>((const double*)f, geo, even, b, c, nn);
+                get_macros_f64_kernel<<<blocks, kMacroThreads, 0, s>>>((const double*)f, geo, even, dv, b, c, nn);
             else
                 return cudaErrorInvalidValue;
             return cudaGetLastError();

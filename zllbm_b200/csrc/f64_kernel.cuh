@@ -45,24 +45,6 @@ struct DivByConstant {
     }
 };
 
-// Box cells of a node's neighbours: cell(dx, dy, dz) = bx + ry + rz.
-template <class L> struct NodeCells {
-    int bx[3], ry[3], rz[3];
-    __device__ __forceinline__ NodeCells(const LevelGeom& geo, const Coord& c) {
-#pragma unroll
-        for (int d = -1; d <= 1; ++d) {
-            bx[d + 1] = wrap_or_ghost(c.x[0] + d, geo.n[0], geo.g[0], geo.periodic[0]);
-            ry[d + 1] = geo.a[0] * wrap_or_ghost(c.x[1] + d, geo.n[1], geo.g[1], geo.periodic[1]);
-            rz[d + 1] = L::kDims == 3
-                            ? geo.a[0] * geo.a[1] * wrap_or_ghost(c.x[2] + d, geo.n[2], geo.g[2], geo.periodic[2])
-                            : 0;
-        }
-    }
-    __device__ __forceinline__ int operator()(int dx, int dy, int dz) const {
-        return bx[dx + 1] + ry[dy + 1] + rz[dz + 1];
-    }
-};
-
 // Guo forcing term of direction q (CalForcingTerming2D / 3D, lbm_solver_interface.cpp:443-470); the
 // products with a zero lattice component are left out.
 template <class L>
