@@ -31,13 +31,37 @@ constexpr uint32_t kTmemCols = 256, kColZ1 = 0, kColZ2 = 64, kColDw2 = 128, kCol
 //   MMA5  [dW1 | db1] += dZ1^T [X | 1]
 // with the epilogues (bias, GELU, output, loss, dZ) on the CUDA cores between them.  The weight
 // gradients accumulate in TMEM over the CTA's tiles and are added to `grad` once at the end.
+//
+// Bound by the latency of a tile's chain (five MMA rounds, 128 tanh per thread between them): two CTAs
+// share an SM (TMEM 2 x 256 columns, shared memory 2 x 106 KB) so that one computes while the other
+// waits, each activation's tanh is kept in a register for the backward pass, and the sums of dw3 over a
+// warp's samples are one recursive halving per 16 columns.  37,888 samples with the update, per step: 92 us with
+// one CTA per SM, recomputed tanh and a butterfly per column; 27.5 now.
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
 
-__global__ void __launch_bounds__(128, 1) mlp_train_kernel(const float* __restrict__ net, const float* __restrict__ x,
+// Sums of 16 values over a warp's lanes by recursive halving: 16 shuffles (a butterfly per value: 80).
+// Lane l returns the sum of value (l >> 1).
+__device__ __forceinline__ float warp_sum16(const float* in, int lane) {
+    float v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = in[i];
+#pragma unroll
+    for (int o = 16, n = 8; n > 0; o >>= 1, n >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const float keep = up ? v[n + i] : v[i], give = up ? v[i] : v[n + i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+__global__ void __launch_bounds__(128, 2) mlp_train_kernel(const float* __restrict__ net, const float* __restrict__ x,
                                                            const float* __restrict__ target, long long n, float inv_n,
                                                            float* __restrict__ grad, float* __restrict__ loss,
                                                            int* __restrict__ err) {
@@ -48,6 +72,7 @@ __global__ void __launch_bounds__(128, 1) mlp_train_kernel(const float* __restri
     float* red = fs + 256;  // dw3 [64], db3, loss
     uint64_t* bar = reinterpret_cast<uint64_t*>(sm + kTrBar);
     uint32_t* tbase = reinterpret_cast<uint32_t*>(sm + kTrBar + 8);
+    pdl_wait();
 
     stage_weights(net, sm + kTrW1, sm + kTrW2, w3, b3, mean, istd, sm + kTrA1);
     if (tid < 66) red[tid] = 0.f;
@@ -69,8 +94,9 @@ __global__ void __launch_bounds__(128, 1) mlp_train_kernel(const float* __restri
     const uint32_t sX = tc::smem_u32(sm + kTrX), sA1 = tc::smem_u32(sm + kTrA1), sDz2 = tc::smem_u32(sm + kTrDz2),
                    sDz1 = tc::smem_u32(sm + kTrDz1), sW1 = tc::smem_u32(sm + kTrW1), sW2 = tc::smem_u32(sm + kTrW2);
     uint32_t phase = 0;
-    float loss_acc = 0.f, db3_acc = 0.f;
+    float loss_acc = 0.f, db3_acc = 0.f, dw3_acc[4] = {0.f, 0.f, 0.f, 0.f};
     bool first = true, ok = true;
+    const bool x16 = (reinterpret_cast<uintptr_t>(x) & 15u) == 0;  // 96-byte rows of a 16-byte aligned array
     const long long tiles = (n + kTile - 1) / kTile;
 
     for (long long tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
@@ -78,8 +104,22 @@ __global__ void __launch_bounds__(128, 1) mlp_train_kernel(const float* __restri
         const bool valid = g < n;
         {
             float v[32];
+            if (valid && x16) {
+                const float4* x4 = reinterpret_cast<const float4*>(x + g * kIn);
 #pragma unroll
-            for (int k = 0; k < kIn; ++k) v[k] = valid ? (x[g * kIn + k] - mean[k]) * istd[k] : 0.f;
+                for (int k = 0; k < kIn / 4; ++k) {
+                    const float4 r = __ldg(x4 + k);
+                    v[4 * k] = r.x;
+                    v[4 * k + 1] = r.y;
+                    v[4 * k + 2] = r.z;
+                    v[4 * k + 3] = r.w;
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < kIn; ++k) v[k] = valid ? x[g * kIn + k] : 0.f;
+            }
+#pragma unroll
+            for (int k = 0; k < kIn; ++k) v[k] = valid ? (v[k] - mean[k]) * istd[k] : 0.f;
             v[24] = 1.f;
 #pragma unroll
             for (int k = 25; k < 32; ++k) v[k] = 0.f;
@@ -100,15 +140,13 @@ __global__ void __launch_bounds__(128, 1) mlp_train_kernel(const float* __restri
             tc::commit(bar);
         }
         if (!(ok = wait_mma(bar, phase, err))) break;
+        float th1[kHid], th2[kHid];  // tanh of the two layers' GELUs, for the backward pass
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             float v[16];
             tc::tmem_ld16(tmem + lane_addr + kColZ1 + 16 * c, v);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                float th;
-                v[i] = gelu(v[i], th);
-            }
+            for (int i = 0; i < 16; ++i) v[i] = gelu(v[i], th1[16 * c + i]);
             st_row_chunk(sm + kTrA1, tid, 16 * c, kSboA1, v);
             st_row_chunk(sm + kTrA1, tid, 16 * c + 8, kSboA1, v + 8);
         }
@@ -131,10 +169,7 @@ __global__ void __launch_bounds__(128, 1) mlp_train_kernel(const float* __restri
             float v[16];
             tc::tmem_ld16(tmem + lane_addr + kColZ2 + 16 * c, v);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                float th;
-                y = fmaf(gelu(v[i], th), w3[16 * c + i], y);
-            }
+            for (int i = 0; i < 16; ++i) y = fmaf(gelu(v[i], th2[16 * c + i]), w3[16 * c + i], y);
         }
         const float e = valid ? y - t : 0.f;
         loss_acc = fmaf(e, e, loss_acc);
@@ -142,18 +177,16 @@ __global__ void __launch_bounds__(128, 1) mlp_train_kernel(const float* __restri
         db3_acc += dy;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            float v[16];
+            float v[16], g3[16];
             tc::tmem_ld16(tmem + lane_addr + kColZ2 + 16 * c, v);
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 const int j = 16 * c + i;
-                const float z = v[i];
-                float th;
-                const float a2 = gelu(z, th);
-                const float s = warp_sum(dy * a2);
-                if (lane == 0) atomicAdd(red + j, s);
-                v[i] = dy * w3[j] * gelu_grad(z, th);
+                const float z = v[i], t2 = th2[j];
+                g3[i] = dy * (0.5f * z * (1.f + t2));
+                v[i] = dy * w3[j] * gelu_grad(z, t2);
             }
+            dw3_acc[c] += warp_sum16(g3, lane);
             st_row_chunk(sm + kTrDz2, tid, 16 * c, kSboDz, v);
             st_row_chunk(sm + kTrDz2, tid, 16 * c + 8, kSboDz, v + 8);
         }
@@ -179,12 +212,7 @@ __global__ void __launch_bounds__(128, 1) mlp_train_kernel(const float* __restri
             tc::tmem_ld16(tmem + lane_addr + kColZ2 + 16 * c, da);
             tc::tmem_ld16(tmem + lane_addr + kColZ1 + 16 * c, z1);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const float z = z1[i];
-                float th;
-                gelu(z, th);
-                da[i] *= gelu_grad(z, th);
-            }
+            for (int i = 0; i < 16; ++i) da[i] *= gelu_grad(z1[i], th1[16 * c + i]);
             st_row_chunk(sm + kTrDz1, tid, 16 * c, kSboDz, da);
             st_row_chunk(sm + kTrDz1, tid, 16 * c + 8, kSboDz, da + 8);
         }
@@ -218,11 +246,13 @@ __global__ void __launch_bounds__(128, 1) mlp_train_kernel(const float* __restri
         for (int c = 0; c < 5; ++c) {
             float v[16];
             tc::tmem_ld16(tmem + lane_addr + kColDw2 + 16 * c, v);
+            if (c < 4) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int col = 16 * c + i;
-                if (col < kHid) atomicAdd(grad + oW2 + j * kHid + col, v[i]);
-                else if (col == kHid) atomicAdd(grad + oB2 + j, v[i]);
+                for (int i = 0; i < 16; i += 4)
+                    atomicAdd(reinterpret_cast<float4*>(grad + oW2 + j * kHid + 16 * c + i),
+                              make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]));
+            } else {
+                atomicAdd(grad + oB2 + j, v[0]);
             }
         }
 #pragma unroll
@@ -230,9 +260,11 @@ __global__ void __launch_bounds__(128, 1) mlp_train_kernel(const float* __restri
             float v[16];
             tc::tmem_ld16(tmem + lane_addr + kColDw1 + 16 * c, v);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
+            for (int i = 0; i < 16; i += 4) {
                 const int col = 16 * c + i;
-                if (col < kIn) atomicAdd(grad + oW1 + j * kIn + col, v[i]);
+                if (col < kIn)
+                    atomicAdd(reinterpret_cast<float4*>(grad + oW1 + j * kIn + col),
+                              make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]));
                 else if (col == kIn) atomicAdd(grad + oB1 + j, v[i]);
             }
         }
@@ -242,6 +274,10 @@ __global__ void __launch_bounds__(128, 1) mlp_train_kernel(const float* __restri
     if (lane == 0) {
         atomicAdd(red + 64, db3_acc);
         atomicAdd(red + 65, loss_acc);
+    }
+    if (!(lane & 1)) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) atomicAdd(red + 16 * c + (lane >> 1), dw3_acc[c]);
     }
     tc::fence_before_sync();
     __syncthreads();
@@ -256,11 +292,17 @@ __global__ void __launch_bounds__(128, 1) mlp_train_kernel(const float* __restri
     }
 }
 
+// One Adam update; also clears the gradients and the loss that the next step accumulates into.
 __global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
-                            float* __restrict__ v, int n, float lr, float c1, float c2) {
+                            float* __restrict__ v, int n, float lr, float c1, float c2, float* __restrict__ g_next,
+                            float* __restrict__ loss_next) {
+    pdl_wait();
+    pdl_trigger();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) *loss_next = 0.f;
     if (i >= n) return;
-    const float gi = g[i];
+    g_next[i] = 0.f;
+    const float gi = __ldcg(g + i);
     const float mi = 0.9f * m[i] + 0.1f * gi;
     const float vi = 0.999f * v[i] + 0.001f * gi * gi;
     m[i] = mi;
@@ -534,8 +576,7 @@ __global__ void filter_kernel(const S* __restrict__ f, LevelGeom geo, StepParams
 // The same for factors that divide a warp: a warp takes 32 consecutive nodes of a row of the fine level
 // (coalesced loads; one thread per block strode by the factor), a thread sums the factor^2 nodes of its
 // column in the block, and a butterfly over the factor lanes of a block adds the columns.  The block's
-// lanes share its 29 stores.  256^3 by 4, FP32 (1.4 GB): 585 us with one thread per
-// block, 349 now.
+// lanes share its 29 stores.  256^3 by 4, FP32 (1.4 GB): 585 us with one thread per block, 349 now.
 constexpr int kFilterThreads = 128;
 template <class S>
 __global__ void __launch_bounds__(kFilterThreads) filter_warp_kernel(const S* __restrict__ f, LevelGeom geo, StepParams p,
@@ -886,6 +927,8 @@ struct zl_trainer {
     cudaStream_t own_stream = nullptr;  // the trainer's own stream
     float* w = nullptr;     // kFlat: weights (trainable part first) + normalisation
     float* g = nullptr;     // kTrainable gradients of the last step
+    float* g_next = nullptr;     // gradients and loss of the next step, cleared by the last one
+    float* loss_next = nullptr;
     float* m = nullptr;     // Adam moments
     float* v = nullptr;
     float* loss = nullptr;  // sum of squared errors of the last step
@@ -925,11 +968,15 @@ int zl_trainer_create(const zl_mlp* init, int device, zl_trainer** out) {
     bool ok = cudaStreamCreateWithFlags(&tr->own_stream, cudaStreamNonBlocking) == cudaSuccess &&
               cudaMalloc(&tr->w, sizeof(float) * kFlat) == cudaSuccess &&
               cudaMalloc(&tr->g, sizeof(float) * kTrainable) == cudaSuccess &&
+              cudaMalloc(&tr->g_next, sizeof(float) * kTrainable) == cudaSuccess &&
+              cudaMalloc(&tr->loss_next, sizeof(float)) == cudaSuccess &&
               cudaMalloc(&tr->m, sizeof(float) * kTrainable) == cudaSuccess &&
               cudaMalloc(&tr->v, sizeof(float) * kTrainable) == cudaSuccess &&
               cudaMalloc(&tr->loss, sizeof(float)) == cudaSuccess && cudaMalloc(&tr->err, sizeof(int)) == cudaSuccess;
     ok = ok && cudaMemcpy(tr->w, init, sizeof(float) * kFlat, cudaMemcpyHostToDevice) == cudaSuccess &&
          cudaMemset(tr->g, 0, sizeof(float) * kTrainable) == cudaSuccess &&
+         cudaMemset(tr->g_next, 0, sizeof(float) * kTrainable) == cudaSuccess &&
+         cudaMemset(tr->loss_next, 0, sizeof(float)) == cudaSuccess &&
          cudaMemset(tr->m, 0, sizeof(float) * kTrainable) == cudaSuccess &&
          cudaMemset(tr->v, 0, sizeof(float) * kTrainable) == cudaSuccess &&
          cudaMemset(tr->loss, 0, sizeof(float)) == cudaSuccess && cudaMemset(tr->err, 0, sizeof(int)) == cudaSuccess;
@@ -954,16 +1001,19 @@ int zl_trainer_step(zl_trainer* tr, const float* x_device, const float* y_device
     if (!tr || !x_device || !y_device || n <= 0) return ZL_EINVAL;
     if (cudaSetDevice(tr->device) != cudaSuccess) return ZL_EDEVICE;
     cudaStream_t s = tr->stream;
-    if (cudaMemsetAsync(tr->g, 0, sizeof(float) * kTrainable, s) != cudaSuccess ||
-        cudaMemsetAsync(tr->loss, 0, sizeof(float), s) != cudaSuccess)
-        return ZL_EDEVICE;
+    // the update of the step before cleared these two; what they held was that step's predecessor's
+    std::swap(tr->g, tr->g_next);
+    std::swap(tr->loss, tr->loss_next);
     const long long tiles = (n + kTile - 1) / kTile;
-    const unsigned grid = (unsigned)(tiles < 148 ? tiles : 148);
-    mlp_train_kernel<<<grid, 128, kTrSmem, s>>>(tr->w, x_device, y_device, n, 1.f / (float)n, tr->g, tr->loss,
-                                                tr->err);
+    const unsigned grid = (unsigned)(tiles < 2 * 148 ? tiles : 2 * 148);
+    if (launch_dependent(mlp_train_kernel, dim3(grid), dim3(128), kTrSmem, s, (const float*)tr->w, x_device, y_device,
+                         (long long)n, 1.f / (float)n, tr->g, tr->loss, tr->err) != cudaSuccess)
+        return ZL_EDEVICE;
     ++tr->t;
     const float c1 = 1.f - powf(0.9f, (float)tr->t), c2 = 1.f - powf(0.999f, (float)tr->t);
-    adam_kernel<<<(kTrainable + 255) / 256, 256, 0, s>>>(tr->w, tr->g, tr->m, tr->v, kTrainable, lr, c1, c2);
+    if (launch_dependent(adam_kernel, dim3((kTrainable + 127) / 128), dim3(128), 0, s, tr->w, (const float*)tr->g, tr->m,
+                         tr->v, kTrainable, lr, c1, c2, tr->g_next, tr->loss_next) != cudaSuccess)
+        return ZL_EDEVICE;
     tr->last_n = n;
     return cudaGetLastError() == cudaSuccess ? ZL_OK : ZL_EDEVICE;
 }
@@ -1009,6 +1059,8 @@ void zl_trainer_destroy(zl_trainer* tr) {
     if (tr->own_stream && tr->own_stream != tr->stream) cudaStreamSynchronize(tr->own_stream);
     cudaFree(tr->w);
     cudaFree(tr->g);
+    cudaFree(tr->g_next);
+    cudaFree(tr->loss_next);
     cudaFree(tr->m);
     cudaFree(tr->v);
     cudaFree(tr->loss);

@@ -23,6 +23,7 @@ constexpr int oW1 = 0, oB1 = oW1 + kHid * kIn, oW2 = oB1 + kHid, oB2 = oW2 + kHi
               oB3 = oW3 + kHid, oMean = oB3 + 1, oInvStd = oMean + kIn, kFlat = oInvStd + kIn;
 constexpr int kTrainable = oMean;
 static_assert(kTrainable == 5825, "parameter count");
+static_assert(oW1 % 4 == 0 && oW2 % 4 == 0 && kIn % 8 == 0 && kHid % 8 == 0, "16-byte rows of weights");
 
 constexpr float kGeluK = 0.7978845608028654f;  // sqrt(2 / pi)
 constexpr float kGeluA = 0.044715f;
@@ -90,26 +91,37 @@ __device__ __forceinline__ void st_row_chunk(uint8_t* tile, uint32_t row, uint32
 }
 
 // Stage [W1 | b1] and [W2 | b2] as BF16 tiles and the FP32 vectors; write this thread's row of
-// A1's constant columns (the ones column and the zero padding).
+// A1's constant columns (the ones column and the zero padding).  Eight weights of a row are two
+// 16-byte loads and one core-matrix row (net comes from cudaMalloc and the rows are 96 and 256 bytes).
+// Loaded past L1: a trainer's update kernel may still run when its next step's launch begins.
 __device__ __forceinline__ void stage_weights(const float* __restrict__ net, uint8_t* w1s, uint8_t* w2s, float* w3,
                                               float* b3, float* mean, float* istd, uint8_t* a1s) {
     const int tid = threadIdx.x, nt = blockDim.x;
-    for (int e = tid; e < kHid * 32; e += nt) {
-        const int j = e >> 5, k = e & 31;
-        const float v = k < kIn ? net[oW1 + j * kIn + k] : (k == kIn ? net[oB1 + j] : 0.f);
-        *reinterpret_cast<__nv_bfloat16*>(w1s + tc::tile_offset(j, k, kSboW1)) = __float2bfloat16_rn(v);
+    auto chunk = [&](uint8_t* tile, uint32_t sbo, int row, int col, const float* src) {
+        const float4 lo = __ldcg(reinterpret_cast<const float4*>(src)), hi = __ldcg(reinterpret_cast<const float4*>(src) + 1);
+        const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        st_row_chunk(tile, row, col, sbo, v);
+    };
+#pragma unroll 4
+    for (int e = tid; e < kHid * 8; e += nt) chunk(w2s, kSboW2, e >> 3, 8 * (e & 7), net + oW2 + 8 * e);
+    for (int e = tid; e < kHid * 3; e += nt) {
+        const int j = e / 3, c = e - 3 * j;
+        chunk(w1s, kSboW1, j, 8 * c, net + oW1 + 8 * e);
     }
-    for (int e = tid; e < kHid * 80; e += nt) {
-        const int j = e / 80, i = e % 80;
-        const float v = i < kHid ? net[oW2 + j * kHid + i] : (i == kHid ? net[oB2 + j] : 0.f);
-        *reinterpret_cast<__nv_bfloat16*>(w2s + tc::tile_offset(j, i, kSboW2)) = __float2bfloat16_rn(v);
+    for (int j = tid; j < kHid; j += nt) {
+        float v[8] = {__ldcg(net + oB1 + j), 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        st_row_chunk(w1s, j, kIn, kSboW1, v);
+        v[0] = __ldcg(net + oB2 + j);
+        st_row_chunk(w2s, j, kHid, kSboW2, v);
+        v[0] = 0.f;
+        st_row_chunk(w2s, j, kHid + 8, kSboW2, v);
     }
-    for (int e = tid; e < kHid; e += nt) w3[e] = net[oW3 + e];
+    for (int e = tid; e < kHid; e += nt) w3[e] = __ldcg(net + oW3 + e);
     for (int e = tid; e < kIn; e += nt) {
-        mean[e] = net[oMean + e];
-        istd[e] = net[oInvStd + e];
+        mean[e] = __ldcg(net + oMean + e);
+        istd[e] = __ldcg(net + oInvStd + e);
     }
-    if (tid == 0) *b3 = net[oB3];
+    if (tid == 0) *b3 = __ldcg(net + oB3);
     float v[8] = {1.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     st_row_chunk(a1s, tid, 64, kSboA1, v);
     v[0] = 0.f;
