@@ -18,25 +18,32 @@ namespace zl {
 namespace closure {
 
 // ---------------------------------------------------------------- training
-// Shared memory of the training kernel (bytes)
-constexpr uint32_t kTrX = 0, kTrA1 = kTrX + kBytesX, kTrDz2 = kTrA1 + kBytesA1, kTrDz1 = kTrDz2 + kBytesDz,
-                   kTrW1 = kTrDz1 + kBytesDz, kTrW2 = kTrW1 + kBytesW1, kTrF = kTrW2 + kBytesW2,
-                   kTrBar = kTrF + 2048, kTrSmem = kTrBar + 64;
-// TMEM columns: Z1 [0, 64), Z2 then dA1 [64, 128), dW2 | db2 [128, 208), dW1 | db1 [208, 240)
-constexpr uint32_t kTmemCols = 256, kColZ1 = 0, kColZ2 = 64, kColDw2 = 128, kColDw1 = 208;
+// Shared memory of the training kernel (bytes): two tiles, the weights, FP32 vectors and sums
+constexpr uint32_t kTrTiles = 2, kTrThreads = kTrTiles * kTile;
+constexpr uint32_t kTrX = 0, kTrA1 = kTrX + kTrTiles * kBytesX, kTrDz2 = kTrA1 + kTrTiles * kBytesA1,
+                   kTrDz1 = kTrDz2 + kTrTiles * kBytesDz, kTrW1 = kTrDz1 + kTrTiles * kBytesDz, kTrW2 = kTrW1 + kBytesW1,
+                   kTrF = kTrW2 + kBytesW2, kTrSums = kTrF + 2048, kTrBar = kTrSums + kTrThreads / 32 * kHid * 4,
+                   kTrSmem = kTrBar + 64;
+static_assert(kTrSmem <= 227 * 1024, "one CTA per SM");
+// TMEM columns: per tile Z1, then per tile Z2 (later dA1), then dW2 | db2 (80) and dW1 | db1 (32)
+constexpr uint32_t kTmemCols = 512, kColZ1 = 0, kColZ2 = kTrTiles * 64, kColDw2 = 2 * kTrTiles * 64,
+                   kColDw1 = kColDw2 + 80;
 
-// One CTA of 128 threads per tile of 128 samples (thread = sample = TMEM lane).  Per tile:
+// One CTA of 256 threads takes two tiles of 128 samples at a time (thread = sample = TMEM lane of its
+// tile).  Per tile:
 //   MMA1  Z1 = X W1^T               MMA2  Z2 = A1 W2^T
 //   MMA3  dA1 = dZ2 W2              MMA4  [dW2 | db2] += dZ2^T [A1 | 1]
 //   MMA5  [dW1 | db1] += dZ1^T [X | 1]
 // with the epilogues (bias, GELU, output, loss, dZ) on the CUDA cores between them.  The weight
-// gradients accumulate in TMEM over the CTA's tiles and are added to `grad` once at the end.
+// gradients accumulate in TMEM over the CTA's tiles, one after another, and are added to `grad` once at
+// the end.
 //
-// Bound by the latency of a tile's chain (five MMA rounds, 128 tanh per thread between them): two CTAs
-// share an SM (TMEM 2 x 256 columns, shared memory 2 x 106 KB) so that one computes while the other
-// waits, each activation's tanh is kept in a register for the backward pass, and the sums of dw3 over a
-// warp's samples are one recursive halving per 16 columns.  37,888 samples with the update, per step: 92 us with
-// one CTA per SM, recomputed tanh and a butterfly per column; 27.5 now.
+// Bound by the latency of a tile's chain (five MMA rounds, 128 tanh per thread between them): two tiles
+// share each round's waits, each activation's tanh is kept in a register for the backward pass, and the
+// sums of dw3 over a warp's samples are one recursive halving per 16 columns.  Eight steps of 37,888 samples
+// and the read-back of gradients and weights: 900 us with one tile of 128 threads at a time, recomputed tanh
+// and a butterfly per column, 280 now.  (Two CTAs of one tile per SM instead: 310 us, and other partial sums
+// of the gradients, which BF16 operands carry on from step to step.)
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -61,27 +68,32 @@ __device__ __forceinline__ float warp_sum16(const float* in, int lane) {
     return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
-__global__ void __launch_bounds__(128, 2) mlp_train_kernel(const float* __restrict__ net, const float* __restrict__ x,
-                                                           const float* __restrict__ target, long long n, float inv_n,
-                                                           float* __restrict__ grad, float* __restrict__ loss,
-                                                           int* __restrict__ err) {
+__global__ void __launch_bounds__(kTrThreads, 1) mlp_train_kernel(const float* __restrict__ net,
+                                                                  const float* __restrict__ x,
+                                                                  const float* __restrict__ target, long long n,
+                                                                  float inv_n, float* __restrict__ grad,
+                                                                  float* __restrict__ loss, int* __restrict__ err) {
     extern __shared__ __align__(1024) uint8_t sm[];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, slot = tid / kTile, row = tid & (kTile - 1);
     float* fs = reinterpret_cast<float*>(sm + kTrF);
     float *w3 = fs + 128, *b3 = fs + 192, *mean = fs + 200, *istd = fs + 224;
-    float* red = fs + 256;  // dw3 [64], db3, loss
+    float* red = fs + 256;  // db3, loss
+    float* sums = reinterpret_cast<float*>(sm + kTrSums);  // dw3 of each warp's samples
     uint64_t* bar = reinterpret_cast<uint64_t*>(sm + kTrBar);
     uint32_t* tbase = reinterpret_cast<uint32_t*>(sm + kTrBar + 8);
+    uint8_t *xs = sm + kTrX + slot * kBytesX, *a1s = sm + kTrA1 + slot * kBytesA1, *dz2s = sm + kTrDz2 + slot * kBytesDz,
+            *dz1s = sm + kTrDz1 + slot * kBytesDz;
     pdl_wait();
 
-    stage_weights(net, sm + kTrW1, sm + kTrW2, w3, b3, mean, istd, sm + kTrA1);
-    if (tid < 66) red[tid] = 0.f;
+    stage_weights(net, sm + kTrW1, sm + kTrW2, w3, b3, mean, istd, 1.f);
+    stage_ones(a1s);
+    if (tid < 2) red[tid] = 0.f;
     {
         // the zero halves of the dZ tiles
         const float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         for (int c = 64; c < 128; c += 8) {
-            st_row_chunk(sm + kTrDz2, tid, c, kSboDz, v);
-            st_row_chunk(sm + kTrDz1, tid, c, kSboDz, v);
+            st_row_chunk(dz2s, row, c, kSboDz, v);
+            st_row_chunk(dz1s, row, c, kSboDz, v);
         }
     }
     if (warp == 0) tc::tmem_alloc(tbase, kTmemCols);
@@ -90,18 +102,21 @@ __global__ void __launch_bounds__(128, 2) mlp_train_kernel(const float* __restri
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = *tbase;
-    const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
+    const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
+    const uint32_t z1 = tmem + lane_addr + kColZ1 + 64 * slot, z2 = tmem + lane_addr + kColZ2 + 64 * slot;
     const uint32_t sX = tc::smem_u32(sm + kTrX), sA1 = tc::smem_u32(sm + kTrA1), sDz2 = tc::smem_u32(sm + kTrDz2),
                    sDz1 = tc::smem_u32(sm + kTrDz1), sW1 = tc::smem_u32(sm + kTrW1), sW2 = tc::smem_u32(sm + kTrW2);
     uint32_t phase = 0;
-    float loss_acc = 0.f, db3_acc = 0.f, dw3_acc[4] = {0.f, 0.f, 0.f, 0.f};
+    float loss_acc = 0.f, db3_acc = 0.f, dw3 = 0.f;  // dw3: of column tid, in the first 64 threads
     bool first = true, ok = true;
     const bool x16 = (reinterpret_cast<uintptr_t>(x) & 15u) == 0;  // 96-byte rows of a 16-byte aligned array
     const long long tiles = (n + kTile - 1) / kTile;
 
-    for (long long tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-        const long long g = tile * kTile + tid;
-        const bool valid = g < n;
+    // the CTA's tiles are blockIdx.x + k gridDim.x; two at a time, in that order in the weight gradients
+    for (long long tile0 = blockIdx.x; tile0 < tiles && ok; tile0 += (long long)kTrTiles * gridDim.x) {
+        const int active = tile0 + gridDim.x < tiles ? 2 : 1;
+        const long long g = (tile0 + (long long)slot * gridDim.x) * kTile + row;
+        const bool valid = slot < active && g < n;
         {
             float v[32];
             if (valid && x16) {
@@ -124,7 +139,7 @@ __global__ void __launch_bounds__(128, 2) mlp_train_kernel(const float* __restri
 #pragma unroll
             for (int k = 25; k < 32; ++k) v[k] = 0.f;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) st_row_chunk(sm + kTrX, tid, 8 * c, kSboX, v + 8 * c);
+            for (int c = 0; c < 4; ++c) st_row_chunk(xs, row, 8 * c, kSboX, v + 8 * c);
         }
         const float t = valid ? target[g] : 0.f;
 
@@ -134,9 +149,10 @@ __global__ void __launch_bounds__(128, 2) mlp_train_kernel(const float* __restri
         __syncthreads();
         if (tid == 0) {
             tc::fence_after_sync();
-            for (int s = 0; s < 2; ++s)
-                tc::mma_bf16(tmem + kColZ1, tc::desc_kmajor(sX, kSboX, s), tc::desc_kmajor(sW1, kSboW1, s), kIdescFwd,
-                             s > 0);
+            for (int a = 0; a < active; ++a)
+                for (int s = 0; s < 2; ++s)
+                    tc::mma_bf16(tmem + kColZ1 + 64 * a, tc::desc_kmajor(sX + a * kBytesX, kSboX, s),
+                                 tc::desc_kmajor(sW1, kSboW1, s), kIdescFwd, s > 0);
             tc::commit(bar);
         }
         if (!(ok = wait_mma(bar, phase, err))) break;
@@ -144,11 +160,11 @@ __global__ void __launch_bounds__(128, 2) mlp_train_kernel(const float* __restri
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             float v[16];
-            tc::tmem_ld16(tmem + lane_addr + kColZ1 + 16 * c, v);
+            tc::tmem_ld16(z1 + 16 * c, v);
 #pragma unroll
             for (int i = 0; i < 16; ++i) v[i] = gelu(v[i], th1[16 * c + i]);
-            st_row_chunk(sm + kTrA1, tid, 16 * c, kSboA1, v);
-            st_row_chunk(sm + kTrA1, tid, 16 * c + 8, kSboA1, v + 8);
+            st_row_chunk(a1s, row, 16 * c, kSboA1, v);
+            st_row_chunk(a1s, row, 16 * c + 8, kSboA1, v + 8);
         }
 
         // MMA2: Z2 = [A1 | 1] [W2 | b2]^T
@@ -157,9 +173,10 @@ __global__ void __launch_bounds__(128, 2) mlp_train_kernel(const float* __restri
         __syncthreads();
         if (tid == 0) {
             tc::fence_after_sync();
-            for (int s = 0; s < 5; ++s)
-                tc::mma_bf16(tmem + kColZ2, tc::desc_kmajor(sA1, kSboA1, s), tc::desc_kmajor(sW2, kSboW2, s),
-                             kIdescFwd, s > 0);
+            for (int a = 0; a < active; ++a)
+                for (int s = 0; s < 5; ++s)
+                    tc::mma_bf16(tmem + kColZ2 + 64 * a, tc::desc_kmajor(sA1 + a * kBytesA1, kSboA1, s),
+                                 tc::desc_kmajor(sW2, kSboW2, s), kIdescFwd, s > 0);
             tc::commit(bar);
         }
         if (!(ok = wait_mma(bar, phase, err))) break;
@@ -167,7 +184,7 @@ __global__ void __launch_bounds__(128, 2) mlp_train_kernel(const float* __restri
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             float v[16];
-            tc::tmem_ld16(tmem + lane_addr + kColZ2 + 16 * c, v);
+            tc::tmem_ld16(z2 + 16 * c, v);
 #pragma unroll
             for (int i = 0; i < 16; ++i) y = fmaf(gelu(v[i], th2[16 * c + i]), w3[16 * c + i], y);
         }
@@ -178,17 +195,18 @@ __global__ void __launch_bounds__(128, 2) mlp_train_kernel(const float* __restri
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             float v[16], g3[16];
-            tc::tmem_ld16(tmem + lane_addr + kColZ2 + 16 * c, v);
+            tc::tmem_ld16(z2 + 16 * c, v);
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 const int j = 16 * c + i;
                 const float z = v[i], t2 = th2[j];
-                g3[i] = dy * (0.5f * z * (1.f + t2));
-                v[i] = dy * w3[j] * gelu_grad(z, t2);
+                g3[i] = valid ? dy * (0.5f * z * (1.f + t2)) : 0.f;
+                v[i] = valid ? dy * w3[j] * gelu_grad(z, t2) : 0.f;
             }
-            dw3_acc[c] += warp_sum16(g3, lane);
-            st_row_chunk(sm + kTrDz2, tid, 16 * c, kSboDz, v);
-            st_row_chunk(sm + kTrDz2, tid, 16 * c + 8, kSboDz, v + 8);
+            const float s = warp_sum16(g3, lane);
+            if (!(lane & 1)) sums[warp * kHid + 16 * c + (lane >> 1)] = s;
+            st_row_chunk(dz2s, row, 16 * c, kSboDz, v);
+            st_row_chunk(dz2s, row, 16 * c + 8, kSboDz, v + 8);
         }
 
         // MMA3: dA1 = dZ2 W2 (into the Z2 columns), MMA4: [dW2 | db2] += dZ2^T [A1 | 1]
@@ -197,24 +215,30 @@ __global__ void __launch_bounds__(128, 2) mlp_train_kernel(const float* __restri
         __syncthreads();
         if (tid == 0) {
             tc::fence_after_sync();
-            for (int s = 0; s < 4; ++s)
-                tc::mma_bf16(tmem + kColZ2, tc::desc_kmajor(sDz2, kSboDz, s), tc::desc_mnmajor(sW2, kSboW2, s),
-                             kIdescDa1, s > 0);
-            for (int s = 0; s < 8; ++s)
-                tc::mma_bf16(tmem + kColDw2, tc::desc_mnmajor(sDz2, kSboDz, s), tc::desc_mnmajor(sA1, kSboA1, s),
-                             kIdescDw2, !first || s > 0);
+            for (int a = 0; a < active; ++a) {
+                for (int s = 0; s < 4; ++s)
+                    tc::mma_bf16(tmem + kColZ2 + 64 * a, tc::desc_kmajor(sDz2 + a * kBytesDz, kSboDz, s),
+                                 tc::desc_mnmajor(sW2, kSboW2, s), kIdescDa1, s > 0);
+                for (int s = 0; s < 8; ++s)
+                    tc::mma_bf16(tmem + kColDw2, tc::desc_mnmajor(sDz2 + a * kBytesDz, kSboDz, s),
+                                 tc::desc_mnmajor(sA1 + a * kBytesA1, kSboA1, s), kIdescDw2, !first || a > 0 || s > 0);
+            }
             tc::commit(bar);
+        }
+        if (tid < kHid) {
+            // the warps' dw3 sums in order (behind the barrier above; the next ones are written behind others)
+            for (int w = 0; w < 4 * active; ++w) dw3 += sums[w * kHid + tid];
         }
         if (!(ok = wait_mma(bar, phase, err))) break;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            float da[16], z1[16];
-            tc::tmem_ld16(tmem + lane_addr + kColZ2 + 16 * c, da);
-            tc::tmem_ld16(tmem + lane_addr + kColZ1 + 16 * c, z1);
+            float da[16], z[16];
+            tc::tmem_ld16(z2 + 16 * c, da);
+            tc::tmem_ld16(z1 + 16 * c, z);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) da[i] *= gelu_grad(z1[i], th1[16 * c + i]);
-            st_row_chunk(sm + kTrDz1, tid, 16 * c, kSboDz, da);
-            st_row_chunk(sm + kTrDz1, tid, 16 * c + 8, kSboDz, da + 8);
+            for (int i = 0; i < 16; ++i) da[i] *= gelu_grad(z[i], th1[16 * c + i]);
+            st_row_chunk(dz1s, row, 16 * c, kSboDz, da);
+            st_row_chunk(dz1s, row, 16 * c + 8, kSboDz, da + 8);
         }
 
         // MMA5: [dW1 | db1] += dZ1^T [X | 1]
@@ -223,9 +247,10 @@ __global__ void __launch_bounds__(128, 2) mlp_train_kernel(const float* __restri
         __syncthreads();
         if (tid == 0) {
             tc::fence_after_sync();
-            for (int s = 0; s < 8; ++s)
-                tc::mma_bf16(tmem + kColDw1, tc::desc_mnmajor(sDz1, kSboDz, s), tc::desc_mnmajor(sX, kSboX, s),
-                             kIdescDw1, !first || s > 0);
+            for (int a = 0; a < active; ++a)
+                for (int s = 0; s < 8; ++s)
+                    tc::mma_bf16(tmem + kColDw1, tc::desc_mnmajor(sDz1 + a * kBytesDz, kSboDz, s),
+                                 tc::desc_mnmajor(sX + a * kBytesX, kSboX, s), kIdescDw1, !first || a > 0 || s > 0);
             tc::commit(bar);
         }
         if (!(ok = wait_mma(bar, phase, err))) break;
@@ -272,19 +297,15 @@ __global__ void __launch_bounds__(128, 2) mlp_train_kernel(const float* __restri
     loss_acc = warp_sum(loss_acc);
     db3_acc = warp_sum(db3_acc);
     if (lane == 0) {
-        atomicAdd(red + 64, db3_acc);
-        atomicAdd(red + 65, loss_acc);
-    }
-    if (!(lane & 1)) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) atomicAdd(red + 16 * c + (lane >> 1), dw3_acc[c]);
+        atomicAdd(red, db3_acc);
+        atomicAdd(red + 1, loss_acc);
     }
     tc::fence_before_sync();
     __syncthreads();
-    if (ok && tid < kHid) atomicAdd(grad + oW3 + tid, red[tid]);
+    if (ok && tid < kHid) atomicAdd(grad + oW3 + tid, dw3);
     if (ok && tid == 0) {
-        atomicAdd(grad + oB3, red[64]);
-        atomicAdd(loss, red[65]);
+        atomicAdd(grad + oB3, red[0]);
+        atomicAdd(loss, red[1]);
     }
     if (warp == 0) {
         tc::fence_after_sync();
@@ -311,53 +332,56 @@ __global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ g, 
 }
 
 // ---------------------------------------------------------------- forward (inference)
-// Shared memory of the inference kernels (bytes); TMEM: 64 columns, Z1 then Z2
-constexpr uint32_t kFwX = 0, kFwA1 = kFwX + kBytesX, kFwW1 = kFwA1 + kBytesA1, kFwW2 = kFwW1 + kBytesW1,
-                   kFwF = kFwW2 + kBytesW2, kFwBar = kFwF + 1024, kFwSmem = kFwBar + 64;
-constexpr uint32_t kFwSmemLaunch = kFwSmem;
-constexpr uint32_t kInferCols = 64;
-constexpr int kMaxCtaPerSm = 512 / kInferCols;
+// Shared memory of the inference kernels for N tiles per CTA (bytes); TMEM: 64 columns per tile, Z1 then Z2
+template <int N> struct InferSmem {
+    static constexpr uint32_t kA1 = 0, kW1 = kA1 + N * kBytesA1, kW2 = kW1 + kBytesW1, kF = kW2 + kBytesW2,
+                              kBar = kF + 1024, kBytes = kBar + 64;
+    static constexpr uint32_t kCols = kHid * N;
+    static constexpr int kMaxCtaPerSm = 512 / (kHid * N);
+};
 
 // Set-up shared by the inference kernels: weights staged, TMEM allocated, barrier initialised.
+template <int N>
 __device__ __forceinline__ InferTile infer_setup(uint8_t* sm, const float* net, float*& mean, float*& istd) {
+    using M = InferSmem<N>;
     const int warp = threadIdx.x >> 5;
-    float* fs = reinterpret_cast<float*>(sm + kFwF);
+    float* fs = reinterpret_cast<float*>(sm + M::kF);
     float *w3 = fs + 128, *b3 = fs + 192;
     mean = fs + 200;
     istd = fs + 224;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + kFwBar);
-    uint32_t* tbase = reinterpret_cast<uint32_t*>(sm + kFwBar + 8);
-    stage_weights(net, sm + kFwW1, sm + kFwW2, w3, b3, mean, istd, sm + kFwA1);
-    if (warp == 0) tc::tmem_alloc(tbase, kInferCols);
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + M::kBar);
+    uint32_t* tbase = reinterpret_cast<uint32_t*>(sm + M::kBar + 8);
+    stage_weights(net, sm + M::kW1, sm + M::kW2, w3, b3, mean, istd, 0.5f);
+    for (int t = threadIdx.x / kTile; t < N; t += blockDim.x / kTile) stage_ones(sm + M::kA1 + t * kBytesA1);
+    if (warp == 0) tc::tmem_alloc(tbase, M::kCols);
     if (threadIdx.x == 0) tc::mbar_init(bar, 1);
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     InferTile it;
-    it.a1s = sm + kFwA1;
-    it.sX = tc::smem_u32(sm + kFwX);
-    it.sA1 = tc::smem_u32(sm + kFwA1);
-    it.sW1 = tc::smem_u32(sm + kFwW1);
-    it.sW2 = tc::smem_u32(sm + kFwW2);
+    it.a1s = sm + M::kA1;
+    it.sA1 = tc::smem_u32(sm + M::kA1);
+    it.sW1 = tc::smem_u32(sm + M::kW1);
+    it.sW2 = tc::smem_u32(sm + M::kW2);
     it.tmem = *tbase;
-    it.lane_addr = (uint32_t)(warp * 32) << 16;
+    it.lane_addr = (uint32_t)((warp & 3) * 32) << 16;  // warp w reaches TMEM lanes 32 (w mod 4) ..
     it.bar = bar;
     it.w3 = w3;
     it.b3 = *b3;
     return it;
 }
 
-__device__ __forceinline__ void infer_teardown(const InferTile& it, bool ok, uint32_t phase) {
+template <int N> __device__ __forceinline__ void infer_teardown(const InferTile& it, bool ok, uint32_t phase) {
     if (!ok) tc::mbar_wait(it.bar, phase, kWaitLimit);  // give the tensor cores a last bounded wait
     tc::fence_before_sync();
     __syncthreads();
     if ((threadIdx.x >> 5) == 0) {
         tc::fence_after_sync();
-        tc::tmem_dealloc(it.tmem, kInferCols);
+        tc::tmem_dealloc(it.tmem, InferSmem<N>::kCols);
     }
 }
 
-// Write this thread's normalised feature row [x_hat | 1 | 0] into the X tile.
+// Write this thread's normalised feature row [x_hat | 1 | 0] into a tile's X columns (in its A1 tile).
 __device__ __forceinline__ void write_x_row(uint8_t* xs, const float* x, const float* mean, const float* istd,
                                             bool valid) {
     float v[32];
@@ -367,14 +391,14 @@ __device__ __forceinline__ void write_x_row(uint8_t* xs, const float* x, const f
 #pragma unroll
     for (int k = kIn + 1; k < 32; ++k) v[k] = 0.f;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) st_row_chunk(xs, threadIdx.x, 8 * c, kSboX, v + 8 * c);
+    for (int c = 0; c < 4; ++c) st_row_chunk(xs, threadIdx.x, 8 * c, kSboA1, v + 8 * c);
 }
 
 __global__ void __launch_bounds__(128) mlp_forward_kernel(const float* __restrict__ net, const float* __restrict__ x,
                                                           long long n, float* __restrict__ out, int* __restrict__ err) {
     extern __shared__ __align__(1024) uint8_t sm[];
     float *mean, *istd;
-    const InferTile it = infer_setup(sm, net, mean, istd);
+    const InferTile it = infer_setup<1>(sm, net, mean, istd);
     uint32_t phase = 0;
     bool ok = true;
     const long long tiles = (n + kTile - 1) / kTile;
@@ -384,12 +408,12 @@ __global__ void __launch_bounds__(128) mlp_forward_kernel(const float* __restric
         float xv[kIn];
 #pragma unroll
         for (int k = 0; k < kIn; ++k) xv[k] = valid ? x[g * kIn + k] : 0.f;
-        write_x_row(sm + kFwX, xv, mean, istd, valid);
+        write_x_row(it.a1s, xv, mean, istd, valid);
         float y;
-        if (!(ok = infer_tile(it, phase, err, y))) break;
+        if (!(ok = infer_tiles<1>(it, phase, err, &y))) break;
         if (valid) out[g] = y;
     }
-    infer_teardown(it, ok, phase);
+    infer_teardown<1>(it, ok, phase);
 }
 
 // ---------------------------------------------------------------- full-box I/O, features, filter
@@ -709,102 +733,86 @@ __global__ void pairs_stage2_kernel(Grid3 g, const float* __restrict__ filt, con
 }
 
 // ---------------------------------------------------------------- fused collide-stream with the network
-// The AA step of a full periodic box with the learned closure evaluated inside the collision:
-// one persistent CTA of 128 threads per tile of 128 consecutive nodes; each thread loads its
-// node's populations, writes its features into the X tile, the CTA runs the two tensor-core
-// layers, and each thread relaxes with tau = tau0 + 0.5 (sqrt(tau0^2 + 18 c sqrt(2 Pi:Pi)) - tau0)
-// and streams; c is also stored per node (c_node) for the steps that reuse it.  The grid is the
-// number of CTAs that fit on the GPU (shared memory 37 KiB, TMEM 64 columns per CTA).
-constexpr uint32_t kLsSmemLaunch = kFwSmem;
+// The AA step of a full periodic box with the learned closure evaluated inside the collision: a
+// persistent CTA of 256 threads takes 256 consecutive nodes at a time as two tiles of the two
+// tensor-core layers, one node per thread; a node relaxes with tau = tau0 + 0.5 (sqrt(tau0^2 + 18 c
+// sqrt(2 Pi:Pi)) - tau0), the Smagorinsky collision of fused_collide with C = 18 c, and streams; c is also
+// stored per node (c_node) for the steps that reuse it.
+//
+// Bound by its instructions and the waits between its phases (HBM at an eighth, tensor cores at a
+// twentieth).  The features and the collision come from the pair sums of the populations in closed form,
+// only the populations are kept across the network (the collision forms everything else again, which is
+// cheaper than registers), and the GELU leaves its factor 1/2 to the next layer's weights.  Two tiles per
+// CTA share the weights and each barrier, so that three CTAs of 80 registers (24 warps) fit an SM.  Two
+// nodes per thread as packed FP32 pairs execute a fifth fewer instructions and are slower (16 warps);
+// four CTAs of 64 registers are slower too.
+// us per step, SRT, one tile and one node per thread with per-direction equilibria / now: 33^3 69 / 12.6
+// (the weights' staging), 64^3 89 / 31, 128^3 236 / 184, 256^3 1411 / 1380.
+// The grid is the number of CTAs that fit on the GPU (shared memory 55 KiB, TMEM 128 columns per CTA).
+constexpr int kLsTiles = 2, kLsThreads = kLsTiles * kTile;
 
 template <class S, int Coll, bool Odd>
-__global__ void __launch_bounds__(128, 5) learned_step_kernel(S* __restrict__ f, LevelGeom geo, StepParams p,
-                                                           const float* __restrict__ net, float fallback_c,
-                                                           float* __restrict__ c_node, int* __restrict__ err,
-                                                           FastDiv nx, FastDiv ny) {
+__global__ void __launch_bounds__(kLsThreads, 3) learned_step_kernel(S* __restrict__ f, LevelGeom geo, StepParams p,
+                                                                    const float* __restrict__ net, float fallback_c,
+                                                                    float* __restrict__ c_node, int* __restrict__ err,
+                                                                    BoxDiv dv) {
     using Tb = Tables<D3Q19>;
     using St = Storage<S>;
     extern __shared__ __align__(1024) uint8_t sm[];
     float *mean, *istd;
-    const InferTile it = infer_setup(sm, net, mean, istd);
-    const int tid = threadIdx.x;
-    const float tau0 = (float)p.tau;
-    const long long nn = (long long)geo.n[0] * geo.n[1] * geo.n[2];
-    const long long tiles = (nn + kTile - 1) / kTile;
+    const InferTile it = infer_setup<kLsTiles>(sm, net, mean, istd);
+    const uint32_t tid = threadIdx.x;
+    const uint32_t nn = (uint32_t)geo.n[0] * (uint32_t)geo.n[1] * (uint32_t)geo.n[2];  // fewer than 2^31
     const long long st = geo.stride;
     uint32_t phase = 0;
     bool ok = true;
 
-    for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const long long i = tile * kTile + tid;
+    for (uint32_t base = blockIdx.x * kLsThreads; base < nn; base += gridDim.x * kLsThreads) {
+        const uint32_t i = base + tid;
         const bool valid = i < nn;
-        Coord c;
+        F1 pre[19];
         {
-            // node index -> coordinates (x fastest) by multiply-shift division (the box holds
-            // fewer than 2^31 cells)
-            const uint32_t ii = valid ? (uint32_t)i : 0u;
-            const uint32_t r = nx.div(ii), zq = ny.div(r);
-            c.x[0] = (int)(ii - r * (uint32_t)geo.n[0]);
-            c.x[1] = (int)(r - zq * (uint32_t)geo.n[1]);
-            c.x[2] = (int)zq;
-        }
-        // periodic neighbours of the node (the level wraps on every axis)
-        int bx[3], row[3][3];
-        {
-            int by[3], bz[3];
+            const NodeCells<D3Q19> cell(geo, box_coord(geo, dv, valid ? i : 0u));
 #pragma unroll
-            for (int d = -1; d <= 1; ++d) {
-                bx[d + 1] = wrap_or_ghost(c.x[0] + d, geo.n[0], 0, 1);
-                by[d + 1] = wrap_or_ghost(c.x[1] + d, geo.n[1], 0, 1);
-                bz[d + 1] = wrap_or_ghost(c.x[2] + d, geo.n[2], 0, 1);
+            for (int q = 0; q < 19; ++q) {
+                const int k = Odd && q != 0 ? 1 : 0, plane = k ? Tb::opp(q) : q;
+                pre[q] = {valid ? St::load_raw(f + plane * st + cell(-k * Tb::cx(q), -k * Tb::cy(q), -k * Tb::cz(q))) : 0.f};
             }
-#pragma unroll
-            for (int dy = 0; dy < 3; ++dy)
-#pragma unroll
-                for (int dz = 0; dz < 3; ++dz) row[dy][dz] = geo.a[0] * (by[dy] + geo.a[1] * bz[dz]);
         }
-        auto cell = [&](int dx, int dy, int dz) -> int { return bx[dx + 1] + row[dy + 1][dz + 1]; };
-        const int self = cell(0, 0, 0);
-        float pre[19];
-#pragma unroll
-        for (int q = 0; q < 19; ++q) {
-            if (!valid) pre[q] = 0.f;
-            else if (Odd && q != 0) pre[q] = St::load_raw(f + Tb::opp(q) * st + cell(-Tb::cx(q), -Tb::cy(q), -Tb::cz(q)));
-            else pre[q] = St::load_raw(f + q * st + self);
-        }
-        float pp;  // sqrt(2 Pi:Pi) of the unscaled non-equilibrium part
-        float neq[19], mac[4];
-        feq_neq_dev<D3Q19>(pre, neq, p.scale, p.inv_scale, mac);
         {
-            float x[kIn];
-            features(mac[0], neq, tau0, x, &pp, p.inv_scale);
-            write_x_row(sm + kFwX, x, mean, istd, valid);
+            F1 x[kIn];
+            fused_features(pre, p, (float)p.tau, x);
+            float v[32];
+#pragma unroll
+            for (int j = 0; j < kIn; j += 4) {
+                const float4 m = *reinterpret_cast<const float4*>(mean + j), s = *reinterpret_cast<const float4*>(istd + j);
+                v[j] = (x[j].v - m.x) * s.x;
+                v[j + 1] = (x[j + 1].v - m.y) * s.y;
+                v[j + 2] = (x[j + 2].v - m.z) * s.z;
+                v[j + 3] = (x[j + 3].v - m.w) * s.w;
+            }
+            v[kIn] = 1.f;
+#pragma unroll
+            for (int j = kIn + 1; j < 32; ++j) v[j] = 0.f;
+            uint8_t* tile = it.a1s + (tid / kTile) * kBytesA1;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) st_row_chunk(tile, tid & (kTile - 1), 8 * c, kSboA1, v + 8 * c);
         }
         float y;
-        if (!(ok = infer_tile(it, phase, err, y))) break;
+        if (!(ok = infer_tiles<kLsTiles, 1>(it, phase, err, &y))) break;
         if (!valid) continue;
-        const float cc = isfinite(y) ? kCUnit * fminf(fmaxf(y, 0.f), kYMax) : fallback_c;
-        if (c_node) c_node[self] = cc;
-        const float tau = tau0 + 0.5f * (sqrtf(fmaf(tau0, tau0, 18.f * cc * pp)) - tau0);
-        const float omega = 1.f / tau;
-        float post[19];
-        if (Coll == kSrt) {
-#pragma unroll
-            for (int q = 0; q < 19; ++q) post[q] = fmaf(-omega, neq[q], pre[q]);
-        } else {
-            float lam[19];
-#pragma unroll
-            for (int k = 0; k < 19; ++k)
-                lam[k] = Tb::s(k) > 0. ? ((float)Tb::s(k) - omega) / (float)row_norm2<D3Q19>(k) : 0.f;
-            mrt_d3q19_dev(pre, neq, post, omega, lam);
-        }
+        const float cn = isfinite(y) ? kCUnit * fminf(fmaxf(y, 0.f), kYMax) : fallback_c;
+        F1 post[19];
+        fused_collide<Coll == kMrt, true, false>(pre, post, p, F1{18.f * cn}, (const F1*)nullptr, (F1*)nullptr);
+        const NodeCells<D3Q19> cell(geo, box_coord(geo, dv, i));
+        if (c_node) c_node[cell(0, 0, 0)] = cn;
 #pragma unroll
         for (int q = 0; q < 19; ++q) {
-            if (Odd && q != 0) St::store_raw(f + q * st + cell(Tb::cx(q), Tb::cy(q), Tb::cz(q)), post[q]);
-            else St::store_raw(f + Tb::opp(q) * st + self, post[q]);
+            const int k = Odd && q != 0 ? 1 : 0, plane = k ? q : Tb::opp(q);
+            St::store_raw(f + plane * st + cell(k * Tb::cx(q), k * Tb::cy(q), k * Tb::cz(q)), post[q].v);
         }
     }
-    infer_teardown(it, ok, phase);
+    infer_teardown<kLsTiles>(it, ok, phase);
 }
 
 template <class S>
@@ -813,7 +821,7 @@ static cudaError_t learned_step_s(int coll, bool odd, void* f, const LevelGeom& 
     static int grid[4] = {0, 0, 0, 0};
     auto launch = [&](auto kernel, int slot) -> cudaError_t {
         if (!grid[slot]) {
-            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLsSmemLaunch);
+            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)InferSmem<kLsTiles>::kBytes);
             if (e != cudaSuccess) return e;
             int dev = 0, sms = 0, regs_sm = 0, smem_sm = 0, reserved = 0;
             cudaFuncAttributes fa;
@@ -825,17 +833,17 @@ static cudaError_t learned_step_s(int coll, bool odd, void* f, const LevelGeom& 
                 (e = cudaFuncGetAttributes(&fa, kernel)) != cudaSuccess)
                 return e;
             // resident CTAs per SM from registers (allocated per warp in units of 256), shared
-            // memory, and TMEM (at most 512 / 64 so that no CTA waits for columns)
-            const int regs_cta = 4 * ((fa.numRegs * 32 + 255) / 256 * 256);
-            const int by_regs = regs_cta > 0 ? regs_sm / regs_cta : kMaxCtaPerSm;
-            const int by_smem = smem_sm / (int)(kLsSmemLaunch + fa.sharedSizeBytes + reserved);
+            // memory, and TMEM (512 columns, so that no CTA waits for some)
+            const int regs_cta = kLsThreads / 32 * ((fa.numRegs * 32 + 255) / 256 * 256);
+            const int by_regs = regs_cta > 0 ? regs_sm / regs_cta : InferSmem<kLsTiles>::kMaxCtaPerSm;
+            const int by_smem = smem_sm / (int)(InferSmem<kLsTiles>::kBytes + fa.sharedSizeBytes + reserved);
             int per_sm = by_regs < by_smem ? by_regs : by_smem;
-            per_sm = per_sm < kMaxCtaPerSm ? per_sm : kMaxCtaPerSm;
+            per_sm = per_sm < InferSmem<kLsTiles>::kMaxCtaPerSm ? per_sm : InferSmem<kLsTiles>::kMaxCtaPerSm;
             grid[slot] = sms * (per_sm > 0 ? per_sm : 1);
         }
-        kernel<<<grid[slot], 128, kLsSmemLaunch, s>>>(static_cast<S*>(f), geo, p, net, fallback_c, c_node, err,
-                                                      FastDiv::make((uint32_t)geo.n[0]),
-                                                      FastDiv::make((uint32_t)geo.n[1]));
+        kernel<<<grid[slot], kLsThreads, InferSmem<kLsTiles>::kBytes, s>>>(
+            static_cast<S*>(f), geo, p, net, fallback_c, c_node, err,
+            BoxDiv{FastDiv::make((uint32_t)geo.n[0]), FastDiv::make((uint32_t)geo.n[1])});
         return cudaGetLastError();
     };
     if (coll == kMrt)
@@ -948,7 +956,7 @@ static int train_attr_once(int device) {
         if (cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrSmem) !=
                 cudaSuccess ||
             cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kFwSmemLaunch) != cudaSuccess)
+                                 (int)InferSmem<1>::kBytes) != cudaSuccess)
             return ZL_EDEVICE;
         done[device] = true;
     }
@@ -1005,8 +1013,8 @@ int zl_trainer_step(zl_trainer* tr, const float* x_device, const float* y_device
     std::swap(tr->g, tr->g_next);
     std::swap(tr->loss, tr->loss_next);
     const long long tiles = (n + kTile - 1) / kTile;
-    const unsigned grid = (unsigned)(tiles < 2 * 148 ? tiles : 2 * 148);
-    if (launch_dependent(mlp_train_kernel, dim3(grid), dim3(128), kTrSmem, s, (const float*)tr->w, x_device, y_device,
+    const unsigned grid = (unsigned)(tiles < 148 ? tiles : 148);
+    if (launch_dependent(mlp_train_kernel, dim3(grid), dim3(kTrThreads), kTrSmem, s, (const float*)tr->w, x_device, y_device,
                          (long long)n, 1.f / (float)n, tr->g, tr->loss, tr->err) != cudaSuccess)
         return ZL_EDEVICE;
     ++tr->t;
@@ -1090,7 +1098,7 @@ int zl_mlp_forward(const zl_mlp* net, const float* x_device, int64_t n, float* y
         const long long tiles = (n + kTile - 1) / kTile;
         const long long cap = 148 * 4;  // four CTAs per SM: 4 x 64 TMEM columns and 4 x 37 KiB
         const unsigned grid = (unsigned)(tiles < cap ? tiles : cap);
-        mlp_forward_kernel<<<grid, 128, kFwSmemLaunch, s>>>(w, x_device, n, y_device, err);
+        mlp_forward_kernel<<<grid, 128, InferSmem<1>::kBytes, s>>>(w, x_device, n, y_device, err);
         ok = cudaGetLastError() == cudaSuccess &&
              cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, s) == cudaSuccess &&
              cudaStreamSynchronize(s) == cudaSuccess;

@@ -60,26 +60,25 @@ __device__ __forceinline__ float gelu(float z, float& t) {
     t = tanhf(kGeluK * fmaf(kGeluA * z, z * z, z));
     return 0.5f * z * (1.f + t);
 }
-// Inference: the same GELU on packed BF16 pairs (the result is a BF16 operand anyway):
-// z^2, 1 + a z^2, k z, k z (1 + a z^2), tanh.approx.bf16x2, z/2, z/2 + z/2 t -- every step rounds to
-// BF16 (constants a, k rounded to BF16 too).
-// The constants are BF16 bit patterns (a = 0x3d37, k = 0x3f4c, 1 = 0x3f80, 1/2 = 0x3f00, each in
-// both halves), so that no conversion runs per call.
+// Inference: twice the same GELU on packed BF16 pairs (the result is a BF16 operand anyway):
+// z^2, 1 + a z^2, k z, k z (1 + a z^2), tanh.approx.bf16x2, z + z t -- every step rounds to BF16
+// (constants a, k rounded to BF16 too).  The factor 1/2 that is missing sits in the next layer's
+// weights (W2, w3), where halving is exact.
+// The constants are BF16 bit patterns (a = 0x3d37, k = 0x3f4c, 1 = 0x3f80, each in both halves), so that
+// no conversion runs per call.
 __device__ __forceinline__ __nv_bfloat162 bf16x2_bits(uint32_t b) {
     __nv_bfloat162 v;
     memcpy(&v, &b, 4);
     return v;
 }
-__device__ __forceinline__ uint32_t gelu_bf16x2(float z0, float z1) {
+__device__ __forceinline__ uint32_t gelu2_bf16x2(float z0, float z1) {
     const __nv_bfloat162 z = __floats2bfloat162_rn(z0, z1);
-    const __nv_bfloat162 a = bf16x2_bits(0x3d373d37u), k = bf16x2_bits(0x3f4c3f4cu), one = bf16x2_bits(0x3f803f80u),
-                         half = bf16x2_bits(0x3f003f00u);
+    const __nv_bfloat162 a = bf16x2_bits(0x3d373d37u), k = bf16x2_bits(0x3f4c3f4cu), one = bf16x2_bits(0x3f803f80u);
     const __nv_bfloat162 p = __hfma2(__hmul2(z, z), a, one);
     const __nv_bfloat162 arg = __hmul2(__hmul2(z, k), p);
     uint32_t t;
     asm("tanh.approx.bf16x2 %0, %1;" : "=r"(t) : "r"(*reinterpret_cast<const uint32_t*>(&arg)));
-    const __nv_bfloat162 hz = __hmul2(z, half);
-    const __nv_bfloat162 out = __hfma2(hz, *reinterpret_cast<const __nv_bfloat162*>(&t), hz);
+    const __nv_bfloat162 out = __hfma2(z, *reinterpret_cast<const __nv_bfloat162*>(&t), z);
     return *reinterpret_cast<const uint32_t*>(&out);
 }
 __device__ __forceinline__ float gelu_grad(float z, float t) {
@@ -90,23 +89,23 @@ __device__ __forceinline__ void st_row_chunk(uint8_t* tile, uint32_t row, uint32
     *reinterpret_cast<uint4*>(tile + tc::tile_offset(row, col, sbo)) = tc::pack_bf16x8(v);
 }
 
-// Stage [W1 | b1] and [W2 | b2] as BF16 tiles and the FP32 vectors; write this thread's row of
-// A1's constant columns (the ones column and the zero padding).  Eight weights of a row are two
-// 16-byte loads and one core-matrix row (net comes from cudaMalloc and the rows are 96 and 256 bytes).
+// Stage [W1 | b1] and [W2 | b2] as BF16 tiles and the FP32 vectors.  Eight weights of a row are two 16-byte
+// loads and one core-matrix row (net comes from cudaMalloc and the rows are 96 and 256 bytes).
 // Loaded past L1: a trainer's update kernel may still run when its next step's launch begins.
+// scale multiplies W2 and w3 (inference: 1/2, the factor its GELU leaves out).
 __device__ __forceinline__ void stage_weights(const float* __restrict__ net, uint8_t* w1s, uint8_t* w2s, float* w3,
-                                              float* b3, float* mean, float* istd, uint8_t* a1s) {
+                                              float* b3, float* mean, float* istd, float scale) {
     const int tid = threadIdx.x, nt = blockDim.x;
-    auto chunk = [&](uint8_t* tile, uint32_t sbo, int row, int col, const float* src) {
+    auto chunk = [&](uint8_t* tile, uint32_t sbo, int row, int col, const float* src, float k) {
         const float4 lo = __ldcg(reinterpret_cast<const float4*>(src)), hi = __ldcg(reinterpret_cast<const float4*>(src) + 1);
-        const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+        const float v[8] = {k * lo.x, k * lo.y, k * lo.z, k * lo.w, k * hi.x, k * hi.y, k * hi.z, k * hi.w};
         st_row_chunk(tile, row, col, sbo, v);
     };
 #pragma unroll 4
-    for (int e = tid; e < kHid * 8; e += nt) chunk(w2s, kSboW2, e >> 3, 8 * (e & 7), net + oW2 + 8 * e);
+    for (int e = tid; e < kHid * 8; e += nt) chunk(w2s, kSboW2, e >> 3, 8 * (e & 7), net + oW2 + 8 * e, scale);
     for (int e = tid; e < kHid * 3; e += nt) {
         const int j = e / 3, c = e - 3 * j;
-        chunk(w1s, kSboW1, j, 8 * c, net + oW1 + 8 * e);
+        chunk(w1s, kSboW1, j, 8 * c, net + oW1 + 8 * e, 1.f);
     }
     for (int j = tid; j < kHid; j += nt) {
         float v[8] = {__ldcg(net + oB1 + j), 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -116,12 +115,17 @@ __device__ __forceinline__ void stage_weights(const float* __restrict__ net, uin
         v[0] = 0.f;
         st_row_chunk(w2s, j, kHid + 8, kSboW2, v);
     }
-    for (int e = tid; e < kHid; e += nt) w3[e] = __ldcg(net + oW3 + e);
+    for (int e = tid; e < kHid; e += nt) w3[e] = scale * __ldcg(net + oW3 + e);
     for (int e = tid; e < kIn; e += nt) {
         mean[e] = __ldcg(net + oMean + e);
         istd[e] = __ldcg(net + oInvStd + e);
     }
     if (tid == 0) *b3 = __ldcg(net + oB3);
+}
+
+// This thread's row of an A1 tile's constant columns (the ones column and the zero padding).
+__device__ __forceinline__ void stage_ones(uint8_t* a1s) {
+    const int tid = threadIdx.x & (kTile - 1);
     float v[8] = {1.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     st_row_chunk(a1s, tid, 64, kSboA1, v);
     v[0] = 0.f;
@@ -140,75 +144,87 @@ __device__ __forceinline__ bool wait_mma(uint64_t* bar, uint32_t& phase, int* er
     return !failed;
 }
 
-// Inference of one tile: X (this thread's row written by the caller) -> y of this thread's row.
-// 64 TMEM columns (Z1, then Z2); returns false if a tensor-core wait gave up.
+// Inference of N tiles of 128 rows: X (this thread's row of each tile written by the caller) -> y of this
+// thread's rows.  64 TMEM columns per tile (Z1, then Z2).  A tile's X occupies the first 32 columns of its
+// A1 tile, whose constant columns lie beyond: X is dead once the first product is done, so the tile
+// needs no memory of its own.  Returns false if a tensor-core wait gave up.
+static_assert(tc::extent_kmajor(128, kSboA1, 2) <= kBytesA1, "X in the A1 tile as A (K = 32)");
 struct InferTile {
     uint8_t* a1s;
-    uint32_t sX, sA1, sW1, sW2, tmem, lane_addr;
+    uint32_t sA1, sW1, sW2, tmem, lane_addr;
     uint64_t* bar;
-    const float* w3;
+    const float* w3;  // halved
     float b3;
 };
 
-__device__ __forceinline__ bool infer_tile(const InferTile& it, uint32_t& phase, int* err, float& y) {
-    const int tid = threadIdx.x;
+// R rows per thread: R = N with 128 threads (a thread's rows in all tiles), R = 1 with 128 N threads.
+template <int N, int R = N>
+__device__ __forceinline__ bool infer_tiles(const InferTile& it, uint32_t& phase, int* err, float* y) {
+    const int tid = threadIdx.x, row = tid & (kTile - 1), first = R == N ? 0 : tid / kTile;
     tc::fence_proxy_async();
     tc::fence_before_sync();
     __syncthreads();
     if (tid == 0) {
         tc::fence_after_sync();
-        for (int s = 0; s < 2; ++s)
-            tc::mma_bf16(it.tmem, tc::desc_kmajor(it.sX, kSboX, s), tc::desc_kmajor(it.sW1, kSboW1, s), kIdescFwd,
-                         s > 0);
+        for (int t = 0; t < N; ++t)
+            for (int s = 0; s < 2; ++s)
+                tc::mma_bf16(it.tmem + kHid * t, tc::desc_kmajor(it.sA1 + kBytesA1 * t, kSboA1, s),
+                             tc::desc_kmajor(it.sW1, kSboW1, s), kIdescFwd, s > 0);
         tc::commit(it.bar);
     }
     if (!wait_mma(it.bar, phase, err)) return false;
+    // (the loops over tiles and column halves stay loops: unrolled, the step kernel's body outgrows the
+    // instruction cache, a quarter of its stalls)
+#pragma unroll 1
+    for (int h = 2 * first; h < 2 * (first + R); ++h) {  // half h: tile h / 2, columns 32 (h % 2) ..
+        float v[32];
+        tc::tmem_ld32(it.tmem + it.lane_addr + 32 * h, v);
+        uint8_t* dst = it.a1s + kBytesA1 * (h >> 1) + tc::tile_offset(row, 32 * (h & 1), kSboA1);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        float v[16];
-        tc::tmem_ld16(it.tmem + it.lane_addr + 16 * c, v);
-        uint4 lo, hi;
-        lo.x = gelu_bf16x2(v[0], v[1]);
-        lo.y = gelu_bf16x2(v[2], v[3]);
-        lo.z = gelu_bf16x2(v[4], v[5]);
-        lo.w = gelu_bf16x2(v[6], v[7]);
-        hi.x = gelu_bf16x2(v[8], v[9]);
-        hi.y = gelu_bf16x2(v[10], v[11]);
-        hi.z = gelu_bf16x2(v[12], v[13]);
-        hi.w = gelu_bf16x2(v[14], v[15]);
-        *reinterpret_cast<uint4*>(it.a1s + tc::tile_offset(tid, 16 * c, kSboA1)) = lo;
-        *reinterpret_cast<uint4*>(it.a1s + tc::tile_offset(tid, 16 * c + 8, kSboA1)) = hi;
-    }
-    tc::fence_proxy_async();
-    tc::fence_before_sync();
-    __syncthreads();
-    if (tid == 0) {
-        tc::fence_after_sync();
-        for (int s = 0; s < 5; ++s)
-            tc::mma_bf16(it.tmem, tc::desc_kmajor(it.sA1, kSboA1, s), tc::desc_kmajor(it.sW2, kSboW2, s), kIdescFwd,
-                         s > 0);
-        tc::commit(it.bar);
-    }
-    if (!wait_mma(it.bar, phase, err)) return false;
-    float acc = it.b3;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        float v[16];
-        tc::tmem_ld16(it.tmem + it.lane_addr + 16 * c, v);
-#pragma unroll
-        for (int i = 0; i < 16; i += 4) {
-            // w3 four at a time (one 128-bit shared load, the same address for every thread)
-            const float4 w = *reinterpret_cast<const float4*>(it.w3 + 16 * c + i);
-            const uint32_t g0 = gelu_bf16x2(v[i], v[i + 1]), g1 = gelu_bf16x2(v[i + 2], v[i + 3]);
-            const float2 a0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g0));
-            const float2 a1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g1));
-            acc = fmaf(a0.x, w.x, acc);
-            acc = fmaf(a0.y, w.y, acc);
-            acc = fmaf(a1.x, w.z, acc);
-            acc = fmaf(a1.y, w.w, acc);
+        for (int k = 0; k < 4; ++k) {
+            uint4 o;
+            o.x = gelu2_bf16x2(v[8 * k], v[8 * k + 1]);
+            o.y = gelu2_bf16x2(v[8 * k + 2], v[8 * k + 3]);
+            o.z = gelu2_bf16x2(v[8 * k + 4], v[8 * k + 5]);
+            o.w = gelu2_bf16x2(v[8 * k + 6], v[8 * k + 7]);
+            *reinterpret_cast<uint4*>(dst + 128 * k) = o;
         }
     }
-    y = acc;
+    tc::fence_proxy_async();
+    tc::fence_before_sync();
+    __syncthreads();
+    if (tid == 0) {
+        tc::fence_after_sync();
+        for (int t = 0; t < N; ++t)
+            for (int s = 0; s < 5; ++s)
+                tc::mma_bf16(it.tmem + kHid * t, tc::desc_kmajor(it.sA1 + kBytesA1 * t, kSboA1, s),
+                             tc::desc_kmajor(it.sW2, kSboW2, s), kIdescFwd, s > 0);
+        tc::commit(it.bar);
+    }
+    if (!wait_mma(it.bar, phase, err)) return false;
+    float2 acc = make_float2(it.b3, 0.f);
+#pragma unroll 1
+    for (int h = 2 * first; h < 2 * (first + R); ++h) {
+        float v[32];
+        tc::tmem_ld32(it.tmem + it.lane_addr + 32 * h, v);
+        const float* w3 = it.w3 + 32 * (h & 1);
+#pragma unroll
+        for (int i = 0; i < 32; i += 4) {
+            // w3 four at a time (one 128-bit shared load, the same address for every thread)
+            const float4 w = *reinterpret_cast<const float4*>(w3 + i);
+            const uint32_t g0 = gelu2_bf16x2(v[i], v[i + 1]), g1 = gelu2_bf16x2(v[i + 2], v[i + 3]);
+            const float2 a0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g0));
+            const float2 a1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g1));
+            acc = __ffma2_rn(a0, make_float2(w.x, w.y), acc);
+            acc = __ffma2_rn(a1, make_float2(w.z, w.w), acc);
+        }
+        if (h & 1) {
+#pragma unroll
+            for (int t = 0; t < R; ++t)
+                if ((h >> 1) == first + t) y[t] = acc.x + acc.y;
+            acc = make_float2(it.b3, 0.f);
+        }
+    }
     return true;
 }
 
@@ -278,6 +294,85 @@ __device__ __forceinline__ void features(float rho, const float* neq, float tau0
     const float s2 = sqrtf(2.f * pp);
     x[23] = 0.5f * (sqrtf(tau0 * tau0 + 18.f * kCUnit * s2) - tau0);
     if (spp) *spp = s2;
+}
+
+// The same features of a node (F1) or a node pair (F2) from its deviations d (scaled units), in the closed
+// forms of fused_collide: the relaxed moments and the stress of f - feq from the pair sums of d and the
+// equilibrium's moments, no per-direction feq.  m9 = 2 Pxx - Pyy - Pzz, m11 = Pyy - Pzz, m13..15 the off-diagonal
+// stress.
+template <class V>
+__device__ __forceinline__ void fused_features(const V* d, const StepParams& p, float tau0, V* x) {
+    auto S = [](float s) { return splat_as<V>(s); };
+    const V S1 = d[1] + d[2], D1 = d[1] - d[2];
+    const V S2 = d[3] + d[4], D2 = d[3] - d[4];
+    const V S3 = d[5] + d[6], D3 = d[5] - d[6];
+    const V S4 = d[7] + d[10], D4 = d[7] - d[10];
+    const V S5 = d[8] + d[9], D5 = d[8] - d[9];
+    const V S6 = d[11] + d[14], D6 = d[11] - d[14];
+    const V S7 = d[12] + d[13], D7 = d[12] - d[13];
+    const V S8 = d[15] + d[18], D8 = d[15] - d[18];
+    const V S9 = d[16] + d[17], D9 = d[16] - d[17];
+    const V S23 = S2 + S3, Sa = S1 + S23;
+    const V Sxy = S4 + S5, Sxz = S6 + S7, Syz = S8 + S9;
+    const V Sd = (Sxy + Sxz) + Syz;
+    const V drho = (d[0] + Sa) + Sd;
+    const V X1 = D4 - D5, X2 = D6 - D7, Y1 = D4 + D5, Y2 = D8 - D9, Z1 = D6 + D7, Z2 = D8 + D9;
+    const V X12 = X1 + X2, Y12 = Y1 + Y2, Z12 = Z1 + Z2;
+    const V zero = S(0.f), is = S(p.inv_scale);
+    const V rho = vfma(drho, is, S(1.f));
+    const V r = each(rho, [](float v) { return __frcp_rn(v); });
+    const V k = is * r;  // unscaled over rho
+    const V ux = (D1 + X12) * k, uy = (D2 + Y12) * k, uz = (D3 + Z12) * k;
+    const V ux2 = ux * ux, uy2 = uy * uy, uz2 = uz * uz;
+    const V usq = (ux2 + uy2) + uz2;
+    const V G = S(p.scale) * rho, nG = zero - G, Gu = G * usq, hG = S(0.5f) * G;
+    const V t = drho * S(1.f / 3.f);
+    const V pxx = vfma(nG, ux2, (S1 + (Sxy + Sxz)) - t);
+    const V pyy = vfma(nG, uy2, (S2 + (Sxy + Syz)) - t);
+    const V pzz = vfma(nG, uz2, (S3 + (Sxz + Syz)) - t);
+    const V pxy = vfma(nG, ux * uy, S4 - S5);
+    const V pxz = vfma(nG, ux * uz, S6 - S7);
+    const V pyz = vfma(nG, uy * uz, S8 - S9);
+    // mass and momentum of f - feq vanish: exact zero inputs
+    x[0] = zero;
+    x[3] = zero;
+    x[5] = zero;
+    x[7] = zero;
+    x[1] = (S(19.f) * ((Sd - d[0]) - Gu)) * k;
+    x[2] = vfma(S(5.5f), Gu, vfma(S(9.f), d[0], vfma(S(-7.f), Sa, S(-2.f) * Sd))) * k;
+    x[4] = vfma(S(-10.f / 3.f), D1, S(5.f / 3.f) * X12) * k;
+    x[6] = vfma(S(-10.f / 3.f), D2, S(5.f / 3.f) * Y12) * k;
+    x[8] = vfma(S(-10.f / 3.f), D3, S(5.f / 3.f) * Z12) * k;
+    x[9] = vfma(S(2.f), pxx, zero - (pyy + pzz)) * k;
+    x[10] = vfma(hG, vfma(S(3.f), ux2, zero - usq),
+                 vfma(S(-4.f), S1, vfma(S(2.f), S23, (Sxy + Sxz) - S(2.f) * Syz))) * k;
+    x[11] = (pyy - pzz) * k;
+    x[12] = vfma(hG, uy2 - uz2, vfma(S(2.f), S3 - S2, Sxy - Sxz)) * k;
+    x[13] = pxy * k;
+    x[14] = pyz * k;
+    x[15] = pxz * k;
+    x[16] = (X1 - X2) * k;
+    x[17] = (Y2 - Y1) * k;
+    x[18] = (Z1 - Z2) * k;
+    // strain S = -3 Pi / (2 rho tau0) and its invariants
+    const V ks = S(-1.5f / tau0) * k;
+    const V sxx = ks * pxx, syy = ks * pyy, szz = ks * pzz, sxy = ks * pxy, sxz = ks * pxz, syz = ks * pyz;
+    const V tr = (sxx + syy) + szz, third = tr * S(1.f / 3.f);
+    const V a = sxx - third, b = syy - third, c = szz - third;
+    const V off = vfma(syz, syz, vfma(sxz, sxz, sxy * sxy)), off2 = S(2.f) * off;
+    const V ss = vfma(szz, szz, vfma(syy, syy, vfma(sxx, sxx, off2)));
+    const V sd2 = vfma(c, c, vfma(b, b, vfma(a, a, off2)));
+    const V det = vfma(a, vfma(b, c, zero - syz * syz),
+                       vfma(zero - sxy, vfma(sxy, c, zero - syz * sxz), sxz * vfma(sxy, syz, zero - b * sxz)));
+    const V pp = vfma(pzz, pzz, vfma(pyy, pyy, pxx * pxx));
+    const V po = vfma(pyz, pyz, vfma(pxz, pxz, pxy * pxy));
+    x[19] = tr;
+    x[20] = ss;
+    x[21] = S(3.f) * det;
+    x[22] = each(S(2.f) * sd2, [](float v) { return __fsqrt_rn(v); });
+    const V s2 = each((is * is) * (S(2.f) * vfma(S(2.f), po, pp)), [](float v) { return __fsqrt_rn(v); });
+    const V root = each(vfma(S(18.f * kCUnit), s2, S(tau0 * tau0)), [](float v) { return __fsqrt_rn(v); });
+    x[23] = S(0.5f) * (root - S(tau0));
 }
 
 }  // namespace closure
