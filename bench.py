@@ -271,7 +271,7 @@ def run_reference_arm(args):
 # ---------------------------------------------------------------- GPU arm
 def time_steps(ctx, steps: int, graph: bool = False):
     """Device time of `steps` time steps on the context's stream (CUDA events): zl_step_level
-    per step, or zl_advance replaying the captured two-step graph."""
+    per step, or zl_advance replaying the captured graph of several steps."""
     import torch
     stream = torch.cuda.ExternalStream(ctx.stream())
     start = torch.cuda.Event(enable_timing=True)

@@ -801,7 +801,8 @@ __device__ __forceinline__ void moment_apply(const float* x, const float* coef, 
 
 // Explicit (FP32 storage): the D3Q19 collisions of fused_collide.cuh, whose bits do not depend on how
 // many nodes a thread updates; the 16-bit storages keep the forms above, which their one-node kernel
-// has always rounded with (their pair and row kernels differ from it in rounding).
+// has always rounded with (their pair and row kernels differ from it in rounding), and so do forced MRT
+// levels, which only the one-node kernel steps.
 template <class L, bool Les, bool Explicit>
 __device__ __forceinline__ void collide_dev(const float* d, float* out, const StepParams& p, int coll, float* mac,
                                             const NodeForce* nf, float les_c = 0.f) {
@@ -1066,7 +1067,7 @@ __device__ __forceinline__ void aa_node(S* __restrict__ f, const LevelGeom& geo,
         if constexpr (St::kDeviation) {
             // Smagorinsky constant C: the level's, or 18 c of the learned closure's last evaluation
             const float les_c = Les ? (p.c_node ? 18.f * __ldg(p.c_node + self) : (float)p.les_c) : 0.f;
-            collide_dev<L, Les, sizeof(S) == 4>(pre, post, p, Coll, mac, Forced ? &nf : nullptr, les_c);
+            collide_dev<L, Les, sizeof(S) == 4 && !(Coll == kMrt && Forced)>(pre, post, p, Coll, mac, Forced ? &nf : nullptr, les_c);
         } else {
             collide_exact<L, Les>(pre, post, p, Coll, mac, Forced ? &nf : nullptr);
         }
@@ -1184,7 +1185,7 @@ __device__ __forceinline__ void aa_node_periodic(S* __restrict__ f, const LevelG
     }
     if constexpr (St::kDeviation) {
         const float les_c = Les ? (p.c_node ? 18.f * __ldg(p.c_node + row + x) : (float)p.les_c) : 0.f;
-        collide_dev<L, Les, sizeof(S) == 4>(pre, post, p, Coll, mac, Forced ? &nf : nullptr, les_c);
+        collide_dev<L, Les, sizeof(S) == 4 && !(Coll == kMrt && Forced)>(pre, post, p, Coll, mac, Forced ? &nf : nullptr, les_c);
     } else {
         collide_exact<L, Les>(pre, post, p, Coll, mac, Forced ? &nf : nullptr);
     }
@@ -1337,5 +1338,28 @@ __device__ __forceinline__ long long post_collision_slot(const LevelGeom& geo, c
     const long long bz = L::kDims == 3 ? wrap_or_ghost(c.x[2] + dz, geo.n[2], geo.g[2], geo.periodic[2]) : 0;
     return plane * geo.stride + bx + (long long)geo.a[0] * (by + (long long)geo.a[1] * bz);
 }
+
+// Slots of one node's populations (post_stream_slot, post_collision_slot for populations known at compile
+// time): the neighbours' cells are formed once per node instead of once per population.  The small
+// passes (faces, transfers, immersed boundary) are launched a few times per step and run for
+// microseconds, so fetching the code of 19 unrolled slot computations is a good part of their time.
+template <class L> struct NodeSlots {
+    NodeCells<L> cell;
+    int self;
+    long long stride;
+    bool even;
+    __device__ __forceinline__ NodeSlots(const LevelGeom& geo, const Coord& c, bool even_layout)
+        : cell(geo, c), self(cell(0, 0, 0)), stride(geo.stride), even(even_layout) {}
+    __device__ __forceinline__ long long post_stream(int q) const {
+        using Tb = Tables<L>;
+        if (even && q != 0) return Tb::opp(q) * stride + cell(-Tb::cx(q), -Tb::cy(q), -Tb::cz(q));
+        return q * stride + self;
+    }
+    __device__ __forceinline__ long long post_collision(int o) const {
+        using Tb = Tables<L>;
+        if (even || o == 0) return Tb::opp(o) * stride + self;
+        return o * stride + cell(Tb::cx(o), Tb::cy(o), Tb::cz(o));
+    }
+};
 
 }  // namespace zl

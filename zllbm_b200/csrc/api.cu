@@ -97,13 +97,16 @@ struct zl_ctx {
     Level levels[ZL_MAX_LEVELS];
     std::string last_error;
     DeviceBuffer scratch_flag;  // int error flag for kernels that validate codes
-    // CUDA graph of graph_steps background steps (zl_set_graph)
+    // CUDA graphs of an even number of background steps (zl_set_graph), one per layout of the background
+    // level (an odd number of steps flips it and no other level's)
     bool use_graph = false;
-    cudaGraphExec_t graph_exec = nullptr;
-    int graph_steps = 0;
-    long long graph_generation = -1;
+    struct StepGraph {
+        cudaGraphExec_t exec = nullptr;
+        int steps = 0;
+        long long generation = -1;
+        int layouts = 0;        // bit l: level l's layout when the graph was captured
+    } graphs[2];
     long long generation = 0;   // bumped by every change of levels, interfaces or vertices
-    int graph_layouts = 0;      // bit l: level l's layout when the graph was captured
     DeviceBuffer closure_net;   // zl_mlp of the learned LES closure (zl_set_closure)
     DeviceBuffer closure_err;   // int: a tensor-core wait of the closure step gave up
     int closure_every = 1;      // the network runs on every closure_every-th step of a level
@@ -301,7 +304,8 @@ int zl_destroy(zl_ctx* ctx) {
         l.partial.release();
     }
     ctx->scratch_flag.release();
-    if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
+    for (auto& g : ctx->graphs)
+        if (g.exec) cudaGraphExecDestroy(g.exec);
     for (cudaStream_t& s : ctx->lstream)
         if (s) cudaStreamSynchronize(s), cudaStreamDestroy(s);
     for (cudaStream_t& s : ctx->ibstream)
@@ -1151,11 +1155,11 @@ int zl_advance(zl_ctx* ctx, int steps) {
     // the captured launches bake in every level's current population layout
     int layouts = 0;
     for (int l = 0; l <= ctx->cfg.max_level; ++l) layouts |= ctx->levels[l].even_layout << l;
-    if (!ctx->graph_exec || ctx->graph_generation != ctx->generation || ctx->graph_layouts != layouts ||
-        ctx->graph_steps < want) {
-        if (ctx->graph_exec) {
-            cudaGraphExecDestroy(ctx->graph_exec);
-            ctx->graph_exec = nullptr;
+    auto& g = ctx->graphs[layouts & 1];
+    if (!g.exec || g.generation != ctx->generation || g.layouts != layouts || g.steps < want) {
+        if (g.exec) {
+            cudaGraphExecDestroy(g.exec);
+            g.exec = nullptr;
         }
         cudaGraph_t graph = nullptr;
         long long steps_before[ZL_MAX_LEVELS];
@@ -1171,17 +1175,17 @@ int zl_advance(zl_ctx* ctx, int steps) {
         ZL_CUDA(ctx, e);
         // capture recorded the launches without running them: the host-side layouts went through an
         // even number of steps and are back where they started
-        const cudaError_t ie = cudaGraphInstantiate(&ctx->graph_exec, graph, 0);
+        const cudaError_t ie = cudaGraphInstantiate(&g.exec, graph, 0);
         cudaGraphDestroy(graph);
         ZL_CUDA(ctx, ie);
-        ctx->graph_generation = ctx->generation;
-        ctx->graph_layouts = layouts;
-        ctx->graph_steps = want;
+        g.generation = ctx->generation;
+        g.layouts = layouts;
+        g.steps = want;
     }
     int s = 0;
-    for (; s + ctx->graph_steps <= steps; s += ctx->graph_steps) {
-        ZL_CUDA(ctx, cudaGraphLaunch(ctx->graph_exec, ctx->stream));
-        for (int l : order) ctx->levels[l].steps += ctx->graph_steps;
+    for (; s + g.steps <= steps; s += g.steps) {
+        ZL_CUDA(ctx, cudaGraphLaunch(g.exec, ctx->stream));
+        for (int l : order) ctx->levels[l].steps += g.steps;
     }
     if (s < steps) return advance_direct(ctx, steps - s, order);
     return ZL_OK;

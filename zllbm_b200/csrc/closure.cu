@@ -430,21 +430,7 @@ __device__ __forceinline__ Coord box_coord(const LevelGeom& geo, const BoxDiv& d
     return c;
 }
 
-// Slots of a node's post-stream populations in the given layout (post_stream_slot): the neighbours' rows
-// are formed once per node, not once per population.
-struct StreamSlots {
-    NodeCells<D3Q19> cell;
-    int self;
-    long long stride;
-    int even;
-    __device__ __forceinline__ StreamSlots(const LevelGeom& geo, const Coord& c, int even_layout)
-        : cell(geo, c), self(cell(0, 0, 0)), stride(geo.stride), even(even_layout) {}
-    __device__ __forceinline__ long long operator()(int q) const {
-        using Tb = Tables<D3Q19>;
-        if (even && q != 0) return Tb::opp(q) * stride + cell(-Tb::cx(q), -Tb::cy(q), -Tb::cz(q));
-        return q * stride + self;
-    }
-};
+using StreamSlots = NodeSlots<D3Q19>;
 
 template <class S>
 __global__ void set_equilibrium_kernel(S* __restrict__ f, LevelGeom geo, StepParams p, int even, BoxDiv dv,
@@ -461,14 +447,14 @@ __global__ void set_equilibrium_kernel(S* __restrict__ f, LevelGeom geo, StepPar
         const float w = (float)Tb::w(q);
         // feq - w = w (rho - 1) + w rho (3 cu + 4.5 cu^2 - 1.5 u^2)
         const float d = w * fmaf(r, fmaf(cu, fmaf(4.5f, cu, 3.f), -usq15), r - 1.f);
-        Storage<S>::store(f + slot(q), d, p);
+        Storage<S>::store(f + slot.post_stream(q), d, p);
     }
 }
 
 template <class S>
 __device__ __forceinline__ void load_node(const S* f, const StreamSlots& slot, float* d) {
 #pragma unroll
-    for (int q = 0; q < 19; ++q) d[q] = Storage<S>::load_raw(f + slot(q));
+    for (int q = 0; q < 19; ++q) d[q] = Storage<S>::load_raw(f + slot.post_stream(q));
 }
 
 constexpr int kMacroThreads = 256;
@@ -517,7 +503,7 @@ __global__ void set_equilibrium_f64_kernel(double* __restrict__ f, LevelGeom geo
     double feq[19];
     feq_exact<D3Q19>((double)rho[i], (double)u[i * 3], (double)u[i * 3 + 1], (double)u[i * 3 + 2], feq);
 #pragma unroll
-    for (int q = 0; q < 19; ++q) f[slot(q)] = feq[q];
+    for (int q = 0; q < 19; ++q) f[slot.post_stream(q)] = feq[q];
 }
 
 __global__ void __launch_bounds__(kMacroThreads) get_macros_f64_kernel(const double* __restrict__ f, LevelGeom geo,
@@ -529,7 +515,7 @@ __global__ void __launch_bounds__(kMacroThreads) get_macros_f64_kernel(const dou
         const StreamSlots slot(geo, box_coord(geo, dv, (uint32_t)i), even);
         double v[19], r, ux, uy, uz;
 #pragma unroll
-        for (int q = 0; q < 19; ++q) v[q] = f[slot(q)];
+        for (int q = 0; q < 19; ++q) v[q] = f[slot.post_stream(q)];
         macro_exact<D3Q19>(v, r, ux, uy, uz);
         rho[i] = (float)r;
         w[0] = (float)ux;
@@ -1012,6 +998,13 @@ int zl_trainer_step(zl_trainer* tr, const float* x_device, const float* y_device
     // the update of the step before cleared these two; what they held was that step's predecessor's
     std::swap(tr->g, tr->g_next);
     std::swap(tr->loss, tr->loss_next);
+    // a captured step runs on the same buffers at every replay, so it clears them itself
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess) return ZL_EDEVICE;
+    if (capturing == cudaStreamCaptureStatusActive &&
+        (cudaMemsetAsync(tr->g, 0, sizeof(float) * kTrainable, s) != cudaSuccess ||
+         cudaMemsetAsync(tr->loss, 0, sizeof(float), s) != cudaSuccess))
+        return ZL_EDEVICE;
     const long long tiles = (n + kTile - 1) / kTile;
     const unsigned grid = (unsigned)(tiles < 148 ? tiles : 148);
     if (launch_dependent(mlp_train_kernel, dim3(grid), dim3(kTrThreads), kTrSmem, s, (const float*)tr->w, x_device, y_device,

@@ -1,5 +1,5 @@
 // The fused D3Q19 collisions of the reduced-precision storages, written once for one node (F1) and
-// for a pair of nodes in packed FP32 registers (F2: fma.rn.f32x2 and friends, sm_100).
+// for a pair of nodes in packed FP32 registers (F2 of pair_value.cuh).
 //
 // Every operation is explicit (no product and sum left for the compiler to contract), so a node's
 // result has the same bits whether a kernel updates it alone or as half of a pair, and step kernels
@@ -18,23 +18,12 @@ __device__ __forceinline__ F1 operator-(F1 a, F1 b) { return {__fsub_rn(a.v, b.v
 __device__ __forceinline__ F1 operator*(F1 a, F1 b) { return {__fmul_rn(a.v, b.v)}; }
 __device__ __forceinline__ F1 vfma(F1 a, F1 b, F1 c) { return {__fmaf_rn(a.v, b.v, c.v)}; }
 
-struct F2 {
-    float2 v;
-};
-__device__ __forceinline__ F2 operator+(F2 a, F2 b) { return {__fadd2_rn(a.v, b.v)}; }
-__device__ __forceinline__ F2 operator-(F2 a, F2 b) { return {__ffma2_rn(b.v, make_float2(-1.f, -1.f), a.v)}; }
-__device__ __forceinline__ F2 operator*(F2 a, F2 b) { return {__fmul2_rn(a.v, b.v)}; }
-__device__ __forceinline__ F2 vfma(F2 a, F2 b, F2 c) { return {__ffma2_rn(a.v, b.v, c.v)}; }
+__device__ __forceinline__ F1 neg(F1 a) { return {-a.v}; }
 
 template <class V> __device__ __forceinline__ V splat_as(float s);
 template <> __device__ __forceinline__ F1 splat_as<F1>(float s) { return {s}; }
-template <> __device__ __forceinline__ F2 splat_as<F2>(float s) { return {make_float2(s, s)}; }
-__device__ __forceinline__ F2 splat(float s) { return splat_as<F2>(s); }
-
 // fn applied to every element
 template <class Fn> __device__ __forceinline__ F1 each(F1 a, Fn fn) { return {fn(a.v)}; }
-template <class Fn> __device__ __forceinline__ F2 each(F2 a, Fn fn) { return {make_float2(fn(a.v.x), fn(a.v.y))}; }
-
 // Relaxation frequency of the Smagorinsky model from the stress norm: tau = tau0 + tau_sgs,
 // tau_sgs = (sqrt(tau0^2 + C sqrt(2 Pi:Pi)) - tau0) / 2 (lbm_les_smagorinsky.cpp:22-94).
 __device__ __forceinline__ float smag_omega(float pi2, float c, float tau0) {
@@ -42,10 +31,6 @@ __device__ __forceinline__ float smag_omega(float pi2, float c, float tau0) {
     return __frcp_rn(__fmaf_rn(0.5f, __fsub_rn(s, tau0), tau0));
 }
 __device__ __forceinline__ F1 smag_omega(F1 pi2, F1 c, float tau0) { return {smag_omega(pi2.v, c.v, tau0)}; }
-__device__ __forceinline__ F2 smag_omega(F2 pi2, F2 c, float tau0) {
-    return {make_float2(smag_omega(pi2.v.x, c.v.x, tau0), smag_omega(pi2.v.y, c.v.y, tau0))};
-}
-
 // D3Q19 SRT (also with a body force) or MRT, on the deviations d (scaled units), in one pass: the pair
 // sums and differences of opposite directions give the density, the momentum, the stress and the
 // relaxed moments, and every opposite pair's output is formed from its sum and difference.
@@ -124,7 +109,7 @@ __device__ __forceinline__ void fused_collide(const V* d, V* out, const StepPara
     }
     V om = S(p.omega32);
     if constexpr (Les) {
-        const V t = drho * S(1.f / 3.f), nG = zero - G;
+        const V t = drho * S(1.f / 3.f), nG = neg(G);
         V pxx = vfma(nG, ux2, (S1 + (Sxy + Sxz)) - t);
         V pyy = vfma(nG, uy2, (S2 + (Sxy + Syz)) - t);
         V pzz = vfma(nG, uz2, (S3 + (Sxz + Syz)) - t);
@@ -165,7 +150,7 @@ __device__ __forceinline__ void fused_collide(const V* d, V* out, const StepPara
         const V a6 = rate(6, 1.f) * vfma(S(-10.f / 3.f), D2, S(5.f / 3.f) * Y12);
         const V a8 = rate(8, 1.f) * vfma(S(-10.f / 3.f), D3, S(5.f / 3.f) * Z12);
         const V hG = S(0.5f) * G;
-        const V a10 = rate(10, 1.f) * vfma(hG, vfma(S(3.f), ux2, zero - usq),
+        const V a10 = rate(10, 1.f) * vfma(hG, vfma(S(3.f), ux2, neg(usq)),
                                            vfma(S(-4.f), S1, vfma(S(2.f), S23, (Sxy + Sxz) - S(2.f) * Syz)));
         const V a12 = rate(12, 1.f) * vfma(hG, uy2 - uz2, vfma(S(2.f), S3 - S2, Sxy - Sxz));
         const V a16 = rate(16, 1.f) * (X1 - X2), a17 = rate(17, 1.f) * (Y2 - Y1), a18 = rate(18, 1.f) * (Z1 - Z2);
@@ -236,10 +221,10 @@ __device__ __forceinline__ void fused_collide(const V* d, V* out, const StepPara
         const V g = vfma(om, S(-0.5f), S(1.f)) * S((float)p.dt * p.scale);
         const V g1 = g * S(1.f / 18.f), g2 = g * S(1.f / 36.f), three = S(3.f), nine = S(9.f);
         const V uF3 = three * vfma(uz, F[2], vfma(uy, F[1], ux * F[0]));
-        out[0] = vfma(keep, d[0], vfma(ow0, B, (zero - g * S(1.f / 3.f)) * uF3));
+        out[0] = vfma(keep, d[0], vfma(ow0, B, neg(g * S(1.f / 3.f)) * uF3));
         // a pair with c.u = cu, c.j = cj, c.F = cF, weight factors K, L, o and gw
         auto forced = [&](int q, int o, V Sq, V Dq, V K, V Lw, V ow, V gw, V cu, V cj, V cF) {
-            const V ev = vfma(gw, vfma(nine * cu, cF, zero - uF3), vfma(K, cu * cu, Lw));
+            const V ev = vfma(gw, vfma(nine * cu, cF, neg(uF3)), vfma(K, cu * cu, Lw));
             pair(q, o, Sq, Dq, ev, vfma(gw * three, cF, ow * cj));
         };
         forced(1, 2, S1, D1, K1, L1, o1, g1, ux, jx, F[0]);
@@ -253,24 +238,24 @@ __device__ __forceinline__ void fused_collide(const V* d, V* out, const StepPara
         forced(16, 17, S9, D9, K2, L2, o2, g2, uz - uy, jz - jy, F[2] - F[1]);
         return;
     }
-    if constexpr (Mrt) out[0] = vfma(keep, d[0], vfma(ow0, B, zero - c0));
+    if constexpr (Mrt) out[0] = vfma(keep, d[0], vfma(ow0, B, neg(c0)));
     else out[0] = vfma(keep, d[0], ow0 * B);
     pair(1, 2, S1, D1, less(vfma(K1, ux2, L1), cx), odd(o1, jx, a4x4));
     pair(3, 4, S2, D2, less(vfma(K1, uy2, L1), cy), odd(o1, jy, a6x4));
     pair(5, 6, S3, D3, less(vfma(K1, uz2, L1), cz), odd(o1, jz, a8x4));
     {
         const V P = less(vfma(K2, ux2 + uy2, L2), c_xy), Q = K2x2 * (ux * uy);
-        pair(7, 10, S4, D4, P + Q, odd(o2, jx + jy, zero - (u1 + u2)));
+        pair(7, 10, S4, D4, P + Q, odd(o2, jx + jy, neg(u1 + u2)));
         pair(8, 9, S5, D5, P - Q, odd(o2, jy - jx, u1 - u2));
     }
     {
         const V P = less(vfma(K2, ux2 + uz2, L2), c_xz), Q = K2x2 * (ux * uz);
-        pair(11, 14, S6, D6, P + Q, odd(o2, jx + jz, zero - (v1 + v2)));
+        pair(11, 14, S6, D6, P + Q, odd(o2, jx + jz, neg(v1 + v2)));
         pair(12, 13, S7, D7, P - Q, odd(o2, jz - jx, v1 - v2));
     }
     {
         const V P = less(vfma(K2, uy2 + uz2, L2), c_yz), Q = K2x2 * (uy * uz);
-        pair(15, 18, S8, D8, P + Q, odd(o2, jy + jz, zero - (t1 + t2)));
+        pair(15, 18, S8, D8, P + Q, odd(o2, jy + jz, neg(t1 + t2)));
         pair(16, 17, S9, D9, P - Q, odd(o2, jz - jy, t1 - t2));
     }
 }

@@ -167,8 +167,9 @@ __global__ void ib_touch_kernel(const S* __restrict__ f, LevelGeom geo, StepPara
     const long long cell = nodes[t];
     Coord c = cell_coord(geo, (int)cell);
     T fv[Q];
+    const NodeSlots<L> slot(geo, c, even_layout);
 #pragma unroll
-    for (int q = 0; q < Q; ++q) fv[q] = St::load(f + post_stream_slot<L>(geo, c, q, even_layout), p);
+    for (int q = 0; q < Q; ++q) fv[q] = St::load(f + slot.post_stream(q), p);
     // func_macro_with_force_ with the node's immersed-boundary force set to zero
     double u[3];
     if constexpr (St::kDeviation) {

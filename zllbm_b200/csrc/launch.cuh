@@ -82,11 +82,22 @@ inline bool pair_eligible(int dims, bool bnd, bool masked, const StepParams& p, 
 //   MRT          12.3 / 14.3   19.5 / 19.0   40.0 / 39.0   58.4 / 53.6   435 / 385
 //   SRT + LES    14.4 / 15.5   22.9 / 20.7   47.0 / 40.0   67.7 / 53.7   508 / 389
 //   MRT + LES    18.9 / 18.1   30.6 / 24.1   55.0 / 42.2   77.9 / 55.6   581 / 407
+// and only where the row's pairs fill nine tenths of the lanes launched for them, unless Smagorinsky makes
+// the one-node kernel's instructions the bound (150^3, 75 pairs on 96 lanes: SRT 87 / 92, MRT 94 / 98).
 constexpr long long kPairMinNodes = 3ll << 19, kPairMinNodesLes = 1ll << 19;
+// Threads along x of the pair kernel's default blocks: the widest rows that leave the fewest lanes idle.
+inline int pair_lanes(int n0, int bx) { return (n0 / 2 + bx - 1) / bx * bx; }
+inline int pair_block_x(int n0) {
+    int bx = 128;
+    for (int w = 64; w >= 32; w /= 2)
+        if (pair_lanes(n0, w) < pair_lanes(n0, bx)) bx = w;
+    return bx;
+}
 inline bool pair_default(int dims, const StepParams& p, int elem_bytes, const LevelGeom& geo) {
     return dims == 3 && elem_bytes == 4 && geo.full && geo.periodic[0] && geo.periodic[1] && geo.periodic[2] &&
-           !p.forced && !p.macro && !(geo.n[0] & 1) && !(geo.stride & 1) &&
-           (p.les ? geo.block[0] >= 0 : geo.block[0] == 0) &&
+           !p.forced && !p.macro && !(geo.n[0] & 1) && !(geo.stride & 1) && geo.n[1] <= 65535 &&
+           (p.les ? geo.block[0] >= 0
+                  : geo.block[0] == 0 && 10 * (geo.n[0] / 2) >= 9 * pair_lanes(geo.n[0], pair_block_x(geo.n[0]))) &&
            (long long)geo.n[0] * geo.n[1] * geo.n[2] >= (p.les ? kPairMinNodesLes : kPairMinNodes);
 }
 

@@ -126,8 +126,12 @@ __global__ void neq_face_kernel(S* __restrict__ f, LevelGeom geo, StepParams p, 
         if (!(__ldg(geo.info + inner) & kInfoPresent)) return;
     }
     T fi[Q];
+    {
+        const NodeSlots<L> from(geo, ci, even_layout);
 #pragma unroll
-    for (int q = 0; q < Q; ++q) fi[q] = St::load(f + post_stream_slot<L>(geo, ci, q, even_layout), p);
+        for (int q = 0; q < Q; ++q) fi[q] = St::load(f + from.post_stream(q), p);
+    }
+    const NodeSlots<L> to(geo, c, even_layout);
     // inner node macros through func_macro_ (with the node's forces when the solver has forces)
     double F[3] = {0., 0., 0.};
     if (p.forced) {
@@ -148,7 +152,7 @@ __global__ void neq_face_kernel(S* __restrict__ f, LevelGeom geo, StepParams p, 
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
             const float db = (float)(feq_b[q] - Tables<L>::w(q));
-            St::store(f + post_stream_slot<L>(geo, c, q, even_layout), db + fi[q] - deq[q], p);
+            St::store(f + to.post_stream(q), db + fi[q] - deq[q], p);
         }
     } else {
         double rho, ux, uy, uz, feq[Q];
@@ -156,7 +160,7 @@ __global__ void neq_face_kernel(S* __restrict__ f, LevelGeom geo, StepParams p, 
         feq_exact<L>(rho, ux, uy, uz, feq);
 #pragma unroll
         for (int q = 0; q < Q; ++q)
-            St::store(f + post_stream_slot<L>(geo, c, q, even_layout), (feq_b[q] + fi[q]) - feq[q], p);
+            St::store(f + to.post_stream(q), (feq_b[q] + fi[q]) - feq[q], p);
     }
 }
 
@@ -213,15 +217,22 @@ __global__ void conv_face_kernel(S* __restrict__ f, LevelGeom geo, StepParams p,
     }
     const T u = (T)p.conv_u[face];
     const T one = (T)1;
+    // every load before the first store (see bb_face_kernel)
+    const NodeSlots<L> own(geo, r.c, even_layout), inner(geo, ci, even_layout);
+    T fb[L::kQ], fi[L::kQ];
+    auto enters = [&](int q) {
+        const int ca = axis == 0 ? Tb::cx(q) : (axis == 1 ? Tb::cy(q) : Tb::cz(q));
+        return ca * out < 0;  // enters across this face iff c . n_out < 0
+    };
 #pragma unroll
     for (int q = 1; q < L::kQ; ++q) {
-        const int ca = axis == 0 ? Tb::cx(q) : (axis == 1 ? Tb::cy(q) : Tb::cz(q));
-        if (ca * out >= 0) continue;  // enters across this face iff c . n_out < 0
-        const long long sb = post_stream_slot<L>(geo, r.c, q, even_layout);
-        const T fb = St::load_raw(f + sb);
-        const T fi = St::load_raw(f + post_stream_slot<L>(geo, ci, q, even_layout));
-        St::store_raw(f + sb, (fb + u * fi) / (one + u));
+        if (!enters(q)) continue;
+        fb[q] = St::load_raw(f + own.post_stream(q));
+        fi[q] = St::load_raw(f + inner.post_stream(q));
     }
+#pragma unroll
+    for (int q = 1; q < L::kQ; ++q)
+        if (enters(q)) St::store_raw(f + own.post_stream(q), (fb[q] + u * fi[q]) / (one + u));
 }
 
 // Bounce back as its own pass (lbm_bounce_back.cpp:28-91): f(x, q_in) = f*(x, o) - 6 rho0 w_o (c_o.U),
@@ -234,12 +245,18 @@ __global__ void bb_face_kernel(S* __restrict__ f, LevelGeom geo, StepParams p, i
     using St = Storage<S>;
     const FaceNode fn = face_node<L>(geo, face);
     if (!fn.ok) return;
+    // Every load before the first store: the pass is a few microseconds of latency, and a load behind a
+    // store it might alias waits for a memory round trip per population (516 nodes: 7 us).  The two never
+    // meet: one side is the node's own slots, the other its ghost cells'.
+    const NodeSlots<L> slot(geo, fn.c, even_layout);
+    typename St::T v[L::kQ];
+#pragma unroll
+    for (int q = 1; q < L::kQ; ++q)
+        if (enters_through<L>(q, face)) v[q] = St::load(f + slot.post_collision(bb_source<L>(q, face)), p);
 #pragma unroll
     for (int q = 1; q < L::kQ; ++q) {
         if (!enters_through<L>(q, face)) continue;
-        const int o = bb_source<L>(q, face);
-        const auto v = St::load(f + post_collision_slot<L>(geo, fn.c, o, even_layout), p);
-        St::store(f + post_stream_slot<L>(geo, fn.c, q, even_layout), v - (decltype(v))p.bb_term[face][o], p);
+        St::store(f + slot.post_stream(q), v[q] - (typename St::T)p.bb_term[face][bb_source<L>(q, face)], p);
     }
 }
 
@@ -261,12 +278,14 @@ __global__ void periodic_face_kernel(S* __restrict__ f, LevelGeom geo, StepParam
                              (long long)geo.a[0] * ((other.x[1] + geo.g[1]) + (long long)geo.a[1] * (other.x[2] + geo.g[2]));
         if (!(__ldg(geo.info + oc) & kInfoPresent)) return;
     }
+    const NodeSlots<L> to(geo, fn.c, even_layout), from(geo, other, even_layout);
+    typename St::T v[L::kQ];
 #pragma unroll
-    for (int q = 1; q < L::kQ; ++q) {
-        if (!enters_through<L>(q, face)) continue;
-        St::store(f + post_stream_slot<L>(geo, fn.c, q, even_layout),
-                  St::load(f + post_stream_slot<L>(geo, other, q, even_layout), p), p);
-    }
+    for (int q = 1; q < L::kQ; ++q)
+        if (enters_through<L>(q, face)) v[q] = St::load(f + from.post_stream(q), p);
+#pragma unroll
+    for (int q = 1; q < L::kQ; ++q)
+        if (enters_through<L>(q, face)) St::store(f + to.post_stream(q), v[q], p);
 }
 
 // ---------------------------------------------------------------- coarse <-> fine transfer
@@ -321,14 +340,14 @@ __global__ void c2f_sources_kernel(const S* __restrict__ ff, LevelGeom fgeo, int
     if (u >= st.n_sources) return;
     T g[Q];
     if (st.src_fine[u]) {
-        const Coord c = cell_coord(fgeo, st.src_cell[u]);
+        const NodeSlots<L> slot(fgeo, cell_coord(fgeo, st.src_cell[u]), f_even);
 #pragma unroll
-        for (int q = 0; q < Q; ++q) g[q] = St::load(ff + post_stream_slot<L>(fgeo, c, q, f_even), fp);
+        for (int q = 0; q < Q; ++q) g[q] = St::load(ff + slot.post_stream(q), fp);
     } else {
-        const Coord c = cell_coord(cgeo, st.src_cell[u]);
+        const NodeSlots<L> slot(cgeo, cell_coord(cgeo, st.src_cell[u]), c_even);
         T fcq[Q];
 #pragma unroll
-        for (int q = 0; q < Q; ++q) fcq[q] = St::load(fc + post_stream_slot<L>(cgeo, c, q, c_even), cp);
+        for (int q = 0; q < Q; ++q) fcq[q] = St::load(fc + slot.post_stream(q), cp);
         if constexpr (St::kDeviation) {
             float rho, ux, uy, uz, deq[Q];
             macro_dev<L>(fcq, rho, ux, uy, uz);
@@ -581,10 +600,12 @@ __global__ void scatter_kernel(S* __restrict__ f, LevelGeom geo, StepParams p, L
     // minimum-plane code writes that node; the maximum-plane copy is ignored, so the result
     // does not depend on which of two disagreeing copies a thread happens to write last.
     if (folded) return;
+    const NodeSlots<L> slot(geo, c, even_layout);
+#pragma unroll
     for (int q = 0; q < L::kQ; ++q) {
         double v = fin[i * L::kQ + q];
         if constexpr (St::kDeviation) v -= Tables<L>::w(q);
-        St::store(f + post_stream_slot<L>(geo, c, q, even_layout), (typename St::T)v, p);
+        St::store(f + slot.post_stream(q), (typename St::T)v, p);
     }
 }
 
@@ -604,9 +625,11 @@ __global__ void gather_kernel(const S* __restrict__ f, LevelGeom geo, StepParams
         return;
     }
     T v[Q];
+    const NodeSlots<L> slot(geo, c, even_layout);
 #pragma unroll
-    for (int q = 0; q < Q; ++q) v[q] = St::load(f + post_stream_slot<L>(geo, c, q, even_layout), p);
+    for (int q = 0; q < Q; ++q) v[q] = St::load(f + slot.post_stream(q), p);
     if (fout) {
+#pragma unroll
         for (int q = 0; q < Q; ++q) {
             double x = (double)v[q];
             if constexpr (St::kDeviation) x += Tables<L>::w(q);
@@ -672,9 +695,10 @@ __global__ void __launch_bounds__(256) conservation_partial_kernel(const S* __re
                 if (!(__ldg(geo.info + self) & kInfoPresent)) continue;
             }
             double rho = 0., jx = 0., jy = 0., jz = 0.;
+            const NodeSlots<L> slot(geo, c, even_layout);
 #pragma unroll
             for (int q = 0; q < Q; ++q) {
-                double v = (double)St::load(f + post_stream_slot<L>(geo, c, q, even_layout), p);
+                double v = (double)St::load(f + slot.post_stream(q), p);
                 if constexpr (St::kDeviation) v += Tables<L>::w(q);
                 rho += v;
                 if (Tables<L>::cx(q)) jx += Tables<L>::cx(q) > 0 ? v : -v;

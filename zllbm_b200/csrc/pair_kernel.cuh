@@ -7,6 +7,7 @@
 // one FMA.  Requires an even row length (x0, x0 + 1 in one row, pair accesses aligned).
 #pragma once
 #include "aa_kernel.cuh"
+#include "pair_value.cuh"
 
 namespace zl {
 
