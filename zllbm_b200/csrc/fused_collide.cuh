@@ -22,8 +22,10 @@ __device__ __forceinline__ F1 neg(F1 a) { return {-a.v}; }
 
 template <class V> __device__ __forceinline__ V splat_as(float s);
 template <> __device__ __forceinline__ F1 splat_as<F1>(float s) { return {s}; }
+
 // fn applied to every element
 template <class Fn> __device__ __forceinline__ F1 each(F1 a, Fn fn) { return {fn(a.v)}; }
+
 // Relaxation frequency of the Smagorinsky model from the stress norm: tau = tau0 + tau_sgs,
 // tau_sgs = (sqrt(tau0^2 + C sqrt(2 Pi:Pi)) - tau0) / 2 (lbm_les_smagorinsky.cpp:22-94).
 __device__ __forceinline__ float smag_omega(float pi2, float c, float tau0) {
@@ -31,6 +33,7 @@ __device__ __forceinline__ float smag_omega(float pi2, float c, float tau0) {
     return __frcp_rn(__fmaf_rn(0.5f, __fsub_rn(s, tau0), tau0));
 }
 __device__ __forceinline__ F1 smag_omega(F1 pi2, F1 c, float tau0) { return {smag_omega(pi2.v, c.v, tau0)}; }
+
 // D3Q19 SRT (also with a body force) or MRT, on the deviations d (scaled units), in one pass: the pair
 // sums and differences of opposite directions give the density, the momentum, the stress and the
 // relaxed moments, and every opposite pair's output is formed from its sum and difference.
