@@ -1,10 +1,9 @@
 // Two nodes per thread with packed FP32 pairs (fma.rn.f32x2 and friends, sm_100): the D3Q19 step
 // of a full periodic box in deviation storage.  Thread t updates nodes x0 = 2t and x0 + 1 of a
 // row.  Populations of the two nodes that sit side by side in a plane move as one 32-bit (FP16 /
-// BF16) or 64-bit (FP32) access; the collision runs once on (node a, node b) pairs in the fused
-// form of mrt_d3q19_fused, which halves its arithmetic instructions.  Same formulas as the
-// scalar kernel; roundings can differ where the scalar build contracts a product and a sum into
-// one FMA.  Requires an even row length (x0, x0 + 1 in one row, pair accesses aligned).
+// BF16) or 64-bit (FP32) access; the collision runs once on (node a, node b) pairs in the form of
+// fused_collide.cuh, which halves its arithmetic instructions.  FP32: the one-node kernel's bits; FP16 / BF16:
+// its formulas, in roundings that can differ where the one-node build contracts a product and a sum.  Requires an even row length (x0, x0 + 1 in one row, pair accesses aligned).
 #pragma once
 #include "aa_kernel.cuh"
 #include "pair_value.cuh"
