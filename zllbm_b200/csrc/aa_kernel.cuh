@@ -1321,26 +1321,10 @@ __device__ __forceinline__ long long post_stream_slot(const LevelGeom& geo, cons
     return plane * geo.stride + bx + (long long)geo.a[0] * (by + (long long)geo.a[1] * bz);
 }
 
-// Slot holding the post-collision population f*(x, o) right after a step whose kernel
-// left the given layout: an even step stores it in slot(x, opp(o)), an odd step in slot(x + c_o, o).
-template <class L>
-__device__ __forceinline__ long long post_collision_slot(const LevelGeom& geo, const Coord& c, int o, bool even_layout) {
-    using Tb = Tables<L>;
-    int dx = 0, dy = 0, dz = 0, plane = Tb::opp(o);
-    if (!even_layout && o != 0) {
-        dx = Tb::cx(o);
-        dy = Tb::cy(o);
-        dz = Tb::cz(o);
-        plane = o;
-    }
-    const long long bx = wrap_or_ghost(c.x[0] + dx, geo.n[0], geo.g[0], geo.periodic[0]);
-    const long long by = wrap_or_ghost(c.x[1] + dy, geo.n[1], geo.g[1], geo.periodic[1]);
-    const long long bz = L::kDims == 3 ? wrap_or_ghost(c.x[2] + dz, geo.n[2], geo.g[2], geo.periodic[2]) : 0;
-    return plane * geo.stride + bx + (long long)geo.a[0] * (by + (long long)geo.a[1] * bz);
-}
-
-// Slots of one node's populations (post_stream_slot, post_collision_slot for populations known at compile
-// time): the neighbours' cells are formed once per node instead of once per population.  The small
+// Slots of one node's populations, known at compile time: post_stream as post_stream_slot, and the slot
+// of the post-collision population f*(x, o) right after a step whose kernel left the given layout (an
+// even step stores it in slot(x, opp(o)), an odd step in slot(x + c_o, o)).  The neighbours' cells are
+// formed once per node instead of once per population.  The small
 // passes (faces, transfers, immersed boundary) are launched a few times per step and run for
 // microseconds, so fetching the code of 19 unrolled slot computations is a good part of their time.
 template <class L> struct NodeSlots {
