@@ -313,17 +313,23 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_kernel(const float* _
     }
 }
 
-// One Adam update; also clears the gradients and the loss that the next step accumulates into.
-__global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
-                            float* __restrict__ v, int n, float lr, float c1, float c2, float* __restrict__ g_next,
-                            float* __restrict__ loss_next) {
+// One Adam update from the gradients that the training kernel summed.  It moves them and the loss to the
+// read-out arrays and leaves the sums cleared, so that every step, launched or replayed from a graph, finds
+// them cleared and leaves them so, and no step clears them in a launch of its own.
+__global__ void adam_kernel(float* __restrict__ w, float* __restrict__ g_sum, float* __restrict__ m,
+                            float* __restrict__ v, int n, float lr, float c1, float c2, float* __restrict__ g,
+                            float* __restrict__ loss_sum, float* __restrict__ loss) {
     pdl_wait();
     pdl_trigger();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) *loss_next = 0.f;
+    if (i == 0) {
+        *loss = __ldcg(loss_sum);
+        *loss_sum = 0.f;
+    }
     if (i >= n) return;
-    g_next[i] = 0.f;
-    const float gi = __ldcg(g + i);
+    const float gi = __ldcg(g_sum + i);
+    g_sum[i] = 0.f;
+    g[i] = gi;
     const float mi = 0.9f * m[i] + 0.1f * gi;
     const float vi = 0.999f * v[i] + 0.001f * gi * gi;
     m[i] = mi;
@@ -920,9 +926,10 @@ struct zl_trainer {
     cudaStream_t stream = nullptr;      // stream the trainer issues on
     cudaStream_t own_stream = nullptr;  // the trainer's own stream
     float* w = nullptr;     // kFlat: weights (trainable part first) + normalisation
+    float* g_sum = nullptr;     // a running step's gradients and squared errors, cleared between steps
+    float* loss_sum = nullptr;
+    bool sums_dirty = false;    // a step was not launched whole: the next one clears the sums first
     float* g = nullptr;     // kTrainable gradients of the last step
-    float* g_next = nullptr;     // gradients and loss of the next step, cleared by the last one
-    float* loss_next = nullptr;
     float* m = nullptr;     // Adam moments
     float* v = nullptr;
     float* loss = nullptr;  // sum of squared errors of the last step
@@ -962,15 +969,15 @@ int zl_trainer_create(const zl_mlp* init, int device, zl_trainer** out) {
     bool ok = cudaStreamCreateWithFlags(&tr->own_stream, cudaStreamNonBlocking) == cudaSuccess &&
               cudaMalloc(&tr->w, sizeof(float) * kFlat) == cudaSuccess &&
               cudaMalloc(&tr->g, sizeof(float) * kTrainable) == cudaSuccess &&
-              cudaMalloc(&tr->g_next, sizeof(float) * kTrainable) == cudaSuccess &&
-              cudaMalloc(&tr->loss_next, sizeof(float)) == cudaSuccess &&
+              cudaMalloc(&tr->g_sum, sizeof(float) * kTrainable) == cudaSuccess &&
+              cudaMalloc(&tr->loss_sum, sizeof(float)) == cudaSuccess &&
               cudaMalloc(&tr->m, sizeof(float) * kTrainable) == cudaSuccess &&
               cudaMalloc(&tr->v, sizeof(float) * kTrainable) == cudaSuccess &&
               cudaMalloc(&tr->loss, sizeof(float)) == cudaSuccess && cudaMalloc(&tr->err, sizeof(int)) == cudaSuccess;
     ok = ok && cudaMemcpy(tr->w, init, sizeof(float) * kFlat, cudaMemcpyHostToDevice) == cudaSuccess &&
          cudaMemset(tr->g, 0, sizeof(float) * kTrainable) == cudaSuccess &&
-         cudaMemset(tr->g_next, 0, sizeof(float) * kTrainable) == cudaSuccess &&
-         cudaMemset(tr->loss_next, 0, sizeof(float)) == cudaSuccess &&
+         cudaMemset(tr->g_sum, 0, sizeof(float) * kTrainable) == cudaSuccess &&
+         cudaMemset(tr->loss_sum, 0, sizeof(float)) == cudaSuccess &&
          cudaMemset(tr->m, 0, sizeof(float) * kTrainable) == cudaSuccess &&
          cudaMemset(tr->v, 0, sizeof(float) * kTrainable) == cudaSuccess &&
          cudaMemset(tr->loss, 0, sizeof(float)) == cudaSuccess && cudaMemset(tr->err, 0, sizeof(int)) == cudaSuccess;
@@ -995,26 +1002,27 @@ int zl_trainer_step(zl_trainer* tr, const float* x_device, const float* y_device
     if (!tr || !x_device || !y_device || n <= 0) return ZL_EINVAL;
     if (cudaSetDevice(tr->device) != cudaSuccess) return ZL_EDEVICE;
     cudaStream_t s = tr->stream;
-    // the update of the step before cleared these two; what they held was that step's predecessor's
-    std::swap(tr->g, tr->g_next);
-    std::swap(tr->loss, tr->loss_next);
-    // a captured step runs on the same buffers at every replay, so it clears them itself
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess) return ZL_EDEVICE;
-    if (capturing == cudaStreamCaptureStatusActive &&
-        (cudaMemsetAsync(tr->g, 0, sizeof(float) * kTrainable, s) != cudaSuccess ||
-         cudaMemsetAsync(tr->loss, 0, sizeof(float), s) != cudaSuccess))
-        return ZL_EDEVICE;
+    if (tr->sums_dirty) {
+        if (cudaMemsetAsync(tr->g_sum, 0, sizeof(float) * kTrainable, s) != cudaSuccess ||
+            cudaMemsetAsync(tr->loss_sum, 0, sizeof(float), s) != cudaSuccess)
+            return ZL_EDEVICE;
+        // a captured clear runs only if its graph does
+        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &capturing) != cudaSuccess) return ZL_EDEVICE;
+        tr->sums_dirty = capturing != cudaStreamCaptureStatusNone;
+    }
     const long long tiles = (n + kTile - 1) / kTile;
     const unsigned grid = (unsigned)(tiles < 148 ? tiles : 148);
     if (launch_dependent(mlp_train_kernel, dim3(grid), dim3(kTrThreads), kTrSmem, s, (const float*)tr->w, x_device, y_device,
-                         (long long)n, 1.f / (float)n, tr->g, tr->loss, tr->err) != cudaSuccess)
+                         (long long)n, 1.f / (float)n, tr->g_sum, tr->loss_sum, tr->err) != cudaSuccess)
         return ZL_EDEVICE;
     ++tr->t;
     const float c1 = 1.f - powf(0.9f, (float)tr->t), c2 = 1.f - powf(0.999f, (float)tr->t);
-    if (launch_dependent(adam_kernel, dim3((kTrainable + 127) / 128), dim3(128), 0, s, tr->w, (const float*)tr->g, tr->m,
-                         tr->v, kTrainable, lr, c1, c2, tr->g_next, tr->loss_next) != cudaSuccess)
+    if (launch_dependent(adam_kernel, dim3((kTrainable + 127) / 128), dim3(128), 0, s, tr->w, tr->g_sum, tr->m, tr->v,
+                         kTrainable, lr, c1, c2, tr->g, tr->loss_sum, tr->loss) != cudaSuccess) {
+        tr->sums_dirty = true;
         return ZL_EDEVICE;
+    }
     tr->last_n = n;
     return cudaGetLastError() == cudaSuccess ? ZL_OK : ZL_EDEVICE;
 }
@@ -1060,8 +1068,8 @@ void zl_trainer_destroy(zl_trainer* tr) {
     if (tr->own_stream && tr->own_stream != tr->stream) cudaStreamSynchronize(tr->own_stream);
     cudaFree(tr->w);
     cudaFree(tr->g);
-    cudaFree(tr->g_next);
-    cudaFree(tr->loss_next);
+    cudaFree(tr->g_sum);
+    cudaFree(tr->loss_sum);
     cudaFree(tr->m);
     cudaFree(tr->v);
     cudaFree(tr->loss);
