@@ -12,6 +12,7 @@
 
 #include "closure.cuh"
 #include "closure_launch.cuh"
+#include "persistent_grid.cuh"
 #include "zllbm_b200.h"
 
 namespace zl {
@@ -810,30 +811,14 @@ __global__ void __launch_bounds__(kLsThreads, 3) learned_step_kernel(S* __restri
 template <class S>
 static cudaError_t learned_step_s(int coll, bool odd, void* f, const LevelGeom& geo, const StepParams& p,
                                   const float* net, float fallback_c, float* c_node, int* err, cudaStream_t s) {
-    static int grid[4] = {0, 0, 0, 0};
+    static PersistentGrid grids[4];
     auto launch = [&](auto kernel, int slot) -> cudaError_t {
-        if (!grid[slot]) {
-            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)InferSmem<kLsTiles>::kBytes);
-            if (e != cudaSuccess) return e;
-            int dev = 0, sms = 0, regs_sm = 0, smem_sm = 0, reserved = 0;
-            cudaFuncAttributes fa;
-            if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
-                (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
-                (e = cudaDeviceGetAttribute(&regs_sm, cudaDevAttrMaxRegistersPerMultiprocessor, dev)) != cudaSuccess ||
-                (e = cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev)) != cudaSuccess ||
-                (e = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev)) != cudaSuccess ||
-                (e = cudaFuncGetAttributes(&fa, kernel)) != cudaSuccess)
-                return e;
-            // resident CTAs per SM from registers (allocated per warp in units of 256), shared
-            // memory, and TMEM (512 columns, so that no CTA waits for some)
-            const int regs_cta = kLsThreads / 32 * ((fa.numRegs * 32 + 255) / 256 * 256);
-            const int by_regs = regs_cta > 0 ? regs_sm / regs_cta : InferSmem<kLsTiles>::kMaxCtaPerSm;
-            const int by_smem = smem_sm / (int)(InferSmem<kLsTiles>::kBytes + fa.sharedSizeBytes + reserved);
-            int per_sm = by_regs < by_smem ? by_regs : by_smem;
-            per_sm = per_sm < InferSmem<kLsTiles>::kMaxCtaPerSm ? per_sm : InferSmem<kLsTiles>::kMaxCtaPerSm;
-            grid[slot] = sms * (per_sm > 0 ? per_sm : 1);
-        }
-        kernel<<<grid[slot], kLsThreads, InferSmem<kLsTiles>::kBytes, s>>>(
+        using M = InferSmem<kLsTiles>;
+        int grid = 0;
+        // (TMEM: 512 columns per SM, so that no CTA waits for some)
+        const cudaError_t e = grids[slot].get((const void*)kernel, kLsThreads, (int)M::kBytes, M::kMaxCtaPerSm, &grid);
+        if (e != cudaSuccess) return e;
+        kernel<<<grid, kLsThreads, M::kBytes, s>>>(
             static_cast<S*>(f), geo, p, net, fallback_c, c_node, err,
             BoxDiv{FastDiv::make((uint32_t)geo.n[0]), FastDiv::make((uint32_t)geo.n[1])});
         return cudaGetLastError();
