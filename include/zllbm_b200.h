@@ -223,9 +223,12 @@ int zl_set_batching(zl_ctx* ctx, int enabled);
    amr_project/grid/grid_manager.cpp:997-1023). */
 int zl_set_level_streams(zl_ctx* ctx, int enabled);
 
-/* Replay zl_advance as a captured CUDA graph of an even number of background steps (every launch
-   of the sub-cycled order, transfers and boundary passes included).  The graph is re-captured after any
-   change of levels, interfaces, vertices or tuning.  Off by default. */
+/* Replay zl_advance as captured CUDA graphs of an even number of background steps (every launch
+   of the sub-cycled order, transfers and boundary passes included): pairs of steps, and for a
+   single level up to sixteen once a few hundred steps have been asked for; steps that are one
+   launch each and fill no such graph, and the last of an odd number, are launched directly.  The
+   graphs are re-captured after any change of levels, interfaces, vertices or tuning.  Off by
+   default. */
 int zl_set_graph(zl_ctx* ctx, int enabled);
 
 /* Thread-block shape of a level's step kernel: x (a multiple of 32) by y threads, at most 256;

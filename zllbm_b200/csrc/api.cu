@@ -11,6 +11,7 @@
 #include <vector>
 #include "zllbm_b200.h"
 #include "closure_launch.cuh"
+#include "graph_plan.h"
 #include "topology.cuh"
 #include "vtu.cuh"
 
@@ -97,15 +98,16 @@ struct zl_ctx {
     Level levels[ZL_MAX_LEVELS];
     std::string last_error;
     DeviceBuffer scratch_flag;  // int error flag for kernels that validate codes
-    // CUDA graphs of an even number of background steps (zl_set_graph), one per layout of the background
-    // level (an odd number of steps flips it and no other level's)
+    // CUDA graphs of an even number of background steps (zl_set_graph; graph_plan.h): the pair and the long one
+    // per layout of the background level (an odd number of steps flips it and no other level's)
     bool use_graph = false;
     struct StepGraph {
         cudaGraphExec_t exec = nullptr;
         int steps = 0;
         long long generation = -1;
         int layouts = 0;        // bit l: level l's layout when the graph was captured
-    } graphs[2];
+    } pair_graphs[2], long_graphs[2];
+    long long graph_steps_seen = 0, graph_seen_generation = -1;  // steps asked of graphs since that generation
     long long generation = 0;   // bumped by every change of levels, interfaces or vertices
     DeviceBuffer closure_net;   // zl_mlp of the learned LES closure (zl_set_closure)
     DeviceBuffer closure_err;   // int: a tensor-core wait of the closure step gave up
@@ -304,8 +306,9 @@ int zl_destroy(zl_ctx* ctx) {
         l.partial.release();
     }
     ctx->scratch_flag.release();
-    for (auto& g : ctx->graphs)
-        if (g.exec) cudaGraphExecDestroy(g.exec);
+    for (int k = 0; k < 2; ++k)
+        for (auto* g : {&ctx->pair_graphs[k], &ctx->long_graphs[k]})
+            if (g->exec) cudaGraphExecDestroy(g->exec);
     for (cudaStream_t& s : ctx->lstream)
         if (s) cudaStreamSynchronize(s), cudaStreamDestroy(s);
     for (cudaStream_t& s : ctx->ibstream)
@@ -1121,6 +1124,35 @@ static int advance_direct(zl_ctx* ctx, int steps, const std::vector<int>& order)
     return ZL_OK;
 }
 
+// Captures `steps` (an even number of) background steps into g.
+static int capture_steps(zl_ctx* ctx, int steps, const std::vector<int>& order, int layouts, zl_ctx::StepGraph& g) {
+    if (g.exec) {
+        cudaGraphExecDestroy(g.exec);
+        g.exec = nullptr;
+    }
+    cudaGraph_t graph = nullptr;
+    long long steps_before[ZL_MAX_LEVELS];
+    for (int l = 0; l < ZL_MAX_LEVELS; ++l) steps_before[l] = ctx->levels[l].steps;
+    ZL_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+    const int rc = advance_direct(ctx, steps, order);
+    const cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
+    for (int l = 0; l < ZL_MAX_LEVELS; ++l) ctx->levels[l].steps = steps_before[l];
+    if (rc) {
+        if (graph) cudaGraphDestroy(graph);
+        return rc;
+    }
+    ZL_CUDA(ctx, e);
+    // capture recorded the launches without running them: the host-side layouts went through an
+    // even number of steps and are back where they started
+    const cudaError_t ie = cudaGraphInstantiate(&g.exec, graph, 0);
+    cudaGraphDestroy(graph);
+    ZL_CUDA(ctx, ie);
+    g.generation = ctx->generation;
+    g.layouts = layouts;
+    g.steps = steps;
+    return ZL_OK;
+}
+
 int zl_advance(zl_ctx* ctx, int steps) {
     if (!ctx || steps < 0) return ZL_EINVAL;
     std::vector<int> order;
@@ -1143,52 +1175,33 @@ int zl_advance(zl_ctx* ctx, int steps) {
     // a closure evaluated every k-th step repeats with period k, not with the graph's steps
     const bool periodic_closure = ctx->cfg.les == ZL_LES_LEARNED && ctx->closure_net.ptr && ctx->closure_every > 1;
     if (!ctx->use_graph || steps < 2 || periodic_closure) return advance_direct(ctx, steps, order);
-    // An even number of background steps brings every level back to the same population layout, so one
-    // captured graph replays for any number of its multiples.  Inside a graph the kernels follow one
-    // another as dependent launches, while a graph waits for the one before it, so the graph of a
-    // single level, whose step is one launch, holds up to kGraphSteps steps (65^2 D2Q9 FP64: 4.1 us
-    // per step in graphs of two, 3.1 in graphs of sixteen); a multi-level step is dozens of launches
-    // already.  A call captures no more than it runs, a longer one later captures again (at most up
-    // to kGraphSteps), and steps that fill no graph are launched directly.
-    constexpr int kGraphSteps = 16;
-    const int want = ctx->cfg.max_level > 0 ? 2 : std::min(kGraphSteps, steps & ~1);
     // the captured launches bake in every level's current population layout
     int layouts = 0;
     for (int l = 0; l <= ctx->cfg.max_level; ++l) layouts |= ctx->levels[l].even_layout << l;
-    auto& g = ctx->graphs[layouts & 1];
-    if (!g.exec || g.generation != ctx->generation || g.layouts != layouts || g.steps < want) {
-        if (g.exec) {
-            cudaGraphExecDestroy(g.exec);
-            g.exec = nullptr;
-        }
-        cudaGraph_t graph = nullptr;
-        long long steps_before[ZL_MAX_LEVELS];
-        for (int l = 0; l < ZL_MAX_LEVELS; ++l) steps_before[l] = ctx->levels[l].steps;
-        ZL_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-        const int rc = advance_direct(ctx, want, order);
-        const cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
-        for (int l = 0; l < ZL_MAX_LEVELS; ++l) ctx->levels[l].steps = steps_before[l];
-        if (rc) {
-            if (graph) cudaGraphDestroy(graph);
-            return rc;
-        }
-        ZL_CUDA(ctx, e);
-        // capture recorded the launches without running them: the host-side layouts went through an
-        // even number of steps and are back where they started
-        const cudaError_t ie = cudaGraphInstantiate(&g.exec, graph, 0);
-        cudaGraphDestroy(graph);
-        ZL_CUDA(ctx, ie);
-        g.generation = ctx->generation;
-        g.layouts = layouts;
-        g.steps = want;
+    auto& pair = ctx->pair_graphs[layouts & 1];
+    auto& run = ctx->long_graphs[layouts & 1];
+    auto valid = [&](const zl_ctx::StepGraph& g) {
+        return g.exec && g.generation == ctx->generation && g.layouts == layouts;
+    };
+    if (ctx->graph_seen_generation != ctx->generation) {
+        ctx->graph_seen_generation = ctx->generation;
+        ctx->graph_steps_seen = 0;
     }
-    int s = 0;
-    for (; s + g.steps <= steps; s += g.steps) {
+    const bool single_level = ctx->cfg.max_level == 0;
+    const bool one_launch = single_level && !ctx->levels[0].ordered && ctx->levels[0].n_vertices == 0;
+    const GraphPlan plan = plan_graph(steps, single_level, one_launch, ctx->graph_steps_seen, valid(run) ? run.steps : 0);
+    ctx->graph_steps_seen += steps;
+    int rc;
+    if (plan.runs > 0 && !(valid(run) && run.steps == plan.run) &&
+        (rc = capture_steps(ctx, plan.run, order, layouts, run)))
+        return rc;
+    if (plan.pairs > 0 && !valid(pair) && (rc = capture_steps(ctx, 2, order, layouts, pair))) return rc;
+    for (int k = 0; k < plan.runs + plan.pairs; ++k) {
+        const auto& g = k < plan.runs ? run : pair;
         ZL_CUDA(ctx, cudaGraphLaunch(g.exec, ctx->stream));
         for (int l : order) ctx->levels[l].steps += g.steps;
     }
-    if (s < steps) return advance_direct(ctx, steps - s, order);
-    return ZL_OK;
+    return plan.direct > 0 ? advance_direct(ctx, plan.direct, order) : ZL_OK;
 }
 
 int zl_set_temporal_interpolation(zl_ctx* ctx, int enabled) {
