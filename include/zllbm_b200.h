@@ -233,11 +233,11 @@ int zl_set_graph(zl_ctx* ctx, int enabled);
 
 /* Thread-block shape of a level's step kernel: x (a multiple of 32) by y threads, at most 256;
    a negative x selects the kernel that updates two nodes per thread with packed FP32 pairs
-   (full periodic D3Q19 boxes in FP32/FP16/BF16 storage, no forcing or LES); x = ZL_BLOCK_ROW
-   selects the kernel that gives each warp one whole x-row (y = 1, 2 or 4 rows per block; full
-   periodic D3Q19 boxes in FP16/BF16 storage whose rows hold 128 or 256 nodes, no forcing or
-   LES).  Without a call, large full periodic FP32 boxes take two nodes per thread too (with
-   Smagorinsky whatever the positive shape); in FP32 the two kernels give the same bits. */
+   (full periodic D3Q19 boxes in FP32/FP16/BF16 storage without forcing; with Smagorinsky in FP32
+   with even rows); x = ZL_BLOCK_ROW selects the kernel that gives each warp one whole x-row
+   (y = 1, 2 or 4 rows per block; full periodic D3Q19 boxes in FP16/BF16 storage whose rows hold
+   128 or 256 nodes, no forcing or LES).  Without a call, large full periodic FP32 boxes take two
+   nodes per thread too; in FP32 the two kernels give the same bits. */
 #define ZL_BLOCK_ROW (1 << 20)
 int zl_set_block(zl_ctx* ctx, int level, int x, int y);
 

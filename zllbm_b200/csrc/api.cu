@@ -1238,6 +1238,12 @@ int zl_set_graph(zl_ctx* ctx, int enabled) {
     return ZL_OK;
 }
 
+// Whether the level may take the kernel with two nodes per thread.
+static bool takes_pairs(const zl_ctx* ctx, const Level& L) {
+    return pair_eligible(ctx->dims, L.bnd, L.geo.info != nullptr, L.params, ctx->ops->elem_bytes, L.geo) ||
+           pair_les_eligible(ctx->dims, L.params, ctx->ops->elem_bytes, L.geo);
+}
+
 int zl_set_block(zl_ctx* ctx, int level, int x, int y) {
     int rc = check_level(ctx, level, true);
     if (rc) return rc;
@@ -1255,7 +1261,7 @@ int zl_set_block(zl_ctx* ctx, int level, int x, int y) {
     }
     const int ax = std::abs(x);
     if (ax < 32 || ax % 32 || y < 1 || ax * y > 256) return fail(ctx, ZL_EINVAL, "block shape %d x %d", x, y);
-    if (x < 0 && !pair_eligible(ctx->dims, L.bnd, L.geo.info != nullptr, L.params, ctx->ops->elem_bytes, L.geo))
+    if (x < 0 && !takes_pairs(ctx, L))
         return fail(ctx, ZL_EINVAL, "two nodes per thread needs a full periodic D3Q19 box in reduced storage");
     L.geo.block[0] = x;
     L.geo.block[1] = y;
@@ -1272,12 +1278,12 @@ int zl_autotune(zl_ctx* ctx, int level, int trials, int32_t* chosen) {
     DeviceBuffer saved;
     if ((rc = alloc(ctx, saved, L.f.bytes))) return rc;
     ZL_CUDA(ctx, cudaMemcpyAsync(saved.ptr, L.f.ptr, L.f.bytes, cudaMemcpyDeviceToDevice, ctx->stream));
-    // negative x: two nodes per thread (full periodic D3Q19 boxes in reduced storage only);
+    // negative x: two nodes per thread (takes_pairs);
     // ZL_BLOCK_ROW: one warp per row (FP16/BF16 boxes with 128- or 256-node rows)
     const int shapes[][2] = {{256, 1}, {128, 2}, {128, 1}, {64, 4}, {64, 2}, {32, 8}, {32, 4},
                              {-128, 1}, {-64, 2}, {-256, 1}, {-64, 1},
                              {ZL_BLOCK_ROW, 4}, {ZL_BLOCK_ROW, 2}, {ZL_BLOCK_ROW, 1}};
-    const bool pairs = pair_eligible(ctx->dims, L.bnd, L.geo.info != nullptr, L.params, ctx->ops->elem_bytes, L.geo);
+    const bool pairs = takes_pairs(ctx, L);
     const bool rows = row_eligible(ctx->dims, L.bnd, L.geo.info != nullptr, L.params, ctx->ops->elem_bytes, L.geo);
     cudaEvent_t t0, t1;
     ZL_CUDA(ctx, cudaEventCreate(&t0));

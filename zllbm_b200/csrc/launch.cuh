@@ -70,12 +70,18 @@ inline bool pair_eligible(int dims, bool bnd, bool masked, const StepParams& p, 
     return dims == 3 && (geo.ring || (!bnd && !masked)) && !p.forced && !p.les && elem_bytes < 8;
 }
 
-// Full periodic D3Q19 boxes in FP32 take the two-nodes-per-thread kernel without being asked to, from
-// a size at which its fewer, heavier threads still fill the GPU: with the default block shape, and with
-// Smagorinsky whatever the (positive) shape, which then shapes the pair kernel's blocks.  Its results
-// have the one-node kernel's bits (fused_collide.cuh).  The 16-bit storages keep the kernel that their
-// rounding streams are numbered for.  p.macro: the transfer sources' macros are saved by the masked
+// With Smagorinsky: full periodic FP32 boxes with even rows (the level keeps its per-cell info, so these
+// are dispatched before the masked kernels).  p.macro: the transfer sources' macros are saved by the masked
 // one-node kernel only.
+inline bool pair_les_eligible(int dims, const StepParams& p, int elem_bytes, const LevelGeom& geo) {
+    return dims == 3 && elem_bytes == 4 && p.les && !p.forced && !p.macro && geo.full && geo.periodic[0] &&
+           geo.periodic[1] && geo.periodic[2] && !(geo.n[0] & 1) && !(geo.stride & 1) && geo.n[1] <= 65535;
+}
+
+// Full periodic D3Q19 boxes in FP32 take the two-nodes-per-thread kernel without being asked to (the default
+// block shape), from a size at which its fewer, heavier threads still fill the GPU.  Its results have the
+// one-node kernel's bits (fused_collide.cuh).  The 16-bit storages keep the kernel that their rounding streams
+// are numbered for.
 // Measured us per step, one node / two nodes per thread:
 //                   80^3          96^3          112^3         128^3         256^3
 //   SRT          11.3 / 13.3   16.4 / 18.0   36.3 / 37.5   54.2 / 52.8   403 / 384
@@ -94,11 +100,13 @@ inline int pair_block_x(int n0) {
     return bx;
 }
 inline bool pair_default(int dims, const StepParams& p, int elem_bytes, const LevelGeom& geo) {
-    return dims == 3 && elem_bytes == 4 && geo.full && geo.periodic[0] && geo.periodic[1] && geo.periodic[2] &&
-           !p.forced && !p.macro && !(geo.n[0] & 1) && !(geo.stride & 1) && geo.n[1] <= 65535 &&
-           (p.les ? geo.block[0] >= 0
-                  : geo.block[0] == 0 && 10 * (geo.n[0] / 2) >= 9 * pair_lanes(geo.n[0], pair_block_x(geo.n[0]))) &&
-           (long long)geo.n[0] * geo.n[1] * geo.n[2] >= (p.les ? kPairMinNodesLes : kPairMinNodes);
+    const long long nodes = (long long)geo.n[0] * geo.n[1] * geo.n[2];
+    if (geo.block[0] != 0 || nodes < (p.les ? kPairMinNodesLes : kPairMinNodes)) return false;
+    const int pairs = geo.n[0] / 2, lanes = pair_lanes(geo.n[0], pair_block_x(geo.n[0]));
+    if (p.les) return pair_les_eligible(dims, p, elem_bytes, geo);
+    return 10 * pairs >= 9 * lanes && dims == 3 && elem_bytes == 4 && geo.full && geo.periodic[0] &&
+           geo.periodic[1] && geo.periodic[2] && !p.forced && !p.macro && !(geo.n[0] & 1) && !(geo.stride & 1) &&
+           geo.n[1] <= 65535;
 }
 
 // The one-warp-per-row kernel (row_kernel.cuh): full periodic D3Q19 boxes in 16-bit storage

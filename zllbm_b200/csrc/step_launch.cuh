@@ -34,7 +34,10 @@ cudaError_t launch_one(S* f, const LevelGeom& geo, const StepParams& p, dim3 g, 
 }
 
 template <class S, class L, int C, bool O, bool B, bool M, int X = 0>
-cudaError_t step_one(S* f, const LevelGeom& geo, const StepParams& p, cudaStream_t s) {
+cudaError_t step_one(S* f, const LevelGeom& level, const StepParams& p, cudaStream_t s) {
+    LevelGeom geo = level;
+    // a shape of pairs chosen before the level stopped being one for the pair kernel
+    if (geo.block[0] < 0) geo.block[0] = geo.block[1] = 0;
     dim3 g, b;
     step_shape(geo, L::kDims, g, b);
     const bool default_shape = geo.block[0] == 0 || geo.block[0] == kRowKernelBlockX;
@@ -73,8 +76,6 @@ cudaError_t step_pair(S* f, const LevelGeom& geo, const StepParams& p, cudaStrea
             const int bx = pair_block_x(geo.n[0]);
             pg.block[0] = -bx;
             pg.block[1] = 128 / bx;
-        } else if (geo.block[0] > 0) {
-            pg.block[0] = -geo.block[0];
         }
         dim3 g, b;
         step_shape(pg, 3, g, b);
@@ -109,7 +110,8 @@ cudaError_t step_lco(bool bnd, bool masked, S* f, const LevelGeom& geo, const St
         if (geo.block[0] < 0 && pair_eligible(3, bnd, masked, p, (int)sizeof(S), geo))
             return step_pair<S, C, O, false>(f, geo, p, s);
         if constexpr (sizeof(S) == 4) {
-            if (pair_default(3, p, (int)sizeof(S), geo))
+            if (pair_default(3, p, (int)sizeof(S), geo) ||
+                (geo.block[0] < 0 && pair_les_eligible(3, p, (int)sizeof(S), geo)))
                 return p.les ? step_pair<S, C, O, true>(f, geo, p, s) : step_pair<S, C, O, false>(f, geo, p, s);
         }
     }
