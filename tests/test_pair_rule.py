@@ -38,6 +38,10 @@ int main() {
         }
         for (int block : {-64, 0, 64}) expect(zl::pair_les_eligible(3, les, 4, level(n, n, n, block)), true);
     }
+    // rows that leave lanes idle: 33 of 64 and 45 of 64 never, 23 of 32 and 75 of 96 with Smagorinsky only
+    for (int n : {66, 90}) expect(zl::pair_default(3, les, 4, level(n, 200, 200, 0)), false);
+    for (int n : {46, 150}) expect(zl::pair_default(3, les, 4, level(n, 200, 200, 0)), true);
+    for (int n : {46, 66, 90, 150}) expect(zl::pair_default(3, plain, 4, level(n, 200, 200, 0)), false);
     expect(zl::pair_les_eligible(3, plain, 4, level(128, 128, 128, -64)), false);
     expect(zl::pair_les_eligible(3, les, 4, level(129, 128, 128, -64)), false);
     expect(zl::pair_les_eligible(3, les, 2, level(128, 128, 128, -64)), false);

@@ -88,8 +88,13 @@ inline bool pair_les_eligible(int dims, const StepParams& p, int elem_bytes, con
 //   MRT          12.3 / 14.3   19.5 / 19.0   40.0 / 39.0   58.4 / 53.6   435 / 385
 //   SRT + LES    14.4 / 15.5   22.9 / 20.7   47.0 / 40.0   67.7 / 53.7   508 / 389
 //   MRT + LES    18.9 / 18.1   30.6 / 24.1   55.0 / 42.2   77.9 / 55.6   581 / 407
-// and only where the row's pairs fill nine tenths of the lanes launched for them, unless Smagorinsky makes
-// the one-node kernel's instructions the bound (150^3, 75 pairs on 96 lanes: SRT 87 / 92, MRT 94 / 98).
+// and only where the row's pairs fill enough of the lanes launched for them: nine tenths (150^3, 75 pairs on 96
+// lanes: SRT 87 / 92, MRT 94 / 98), with Smagorinsky, whose one-node kernel is bound by its instructions, five
+// sevenths (one / two nodes per thread, SRT + LES and MRT + LES; share of the lanes in front):
+//   .52  66 x 161 x 150  52.5 / 59.3   59.2 / 63.4       .72  46 x 150 x 150   27.1 / 26.1   34.7 / 29.2
+//   .63  80 x 90 x 90    16.6 / 18.6   20.1 / 21.1       .77  98 x 90 x 90     20.4 / 19.9   24.8 / 21.9
+//   .68  130 x 70 x 70   17.4 / 19.8   20.8 / 21.5       .78  150 x 100 x 100  49.4 / 46.3   55.6 / 48.0
+//   .70  90 x 90 x 90    19.3 / 19.5   23.2 / 21.6       .94  60 x 150 x 150   43.1 / 37.7   50.2 / 38.9
 constexpr long long kPairMinNodes = 3ll << 19, kPairMinNodesLes = 1ll << 19;
 // Threads along x of the pair kernel's default blocks: the widest rows that leave the fewest lanes idle.
 inline int pair_lanes(int n0, int bx) { return (n0 / 2 + bx - 1) / bx * bx; }
@@ -103,7 +108,7 @@ inline bool pair_default(int dims, const StepParams& p, int elem_bytes, const Le
     const long long nodes = (long long)geo.n[0] * geo.n[1] * geo.n[2];
     if (geo.block[0] != 0 || nodes < (p.les ? kPairMinNodesLes : kPairMinNodes)) return false;
     const int pairs = geo.n[0] / 2, lanes = pair_lanes(geo.n[0], pair_block_x(geo.n[0]));
-    if (p.les) return pair_les_eligible(dims, p, elem_bytes, geo);
+    if (p.les) return 7 * pairs >= 5 * lanes && pair_les_eligible(dims, p, elem_bytes, geo);
     return 10 * pairs >= 9 * lanes && dims == 3 && elem_bytes == 4 && geo.full && geo.periodic[0] &&
            geo.periodic[1] && geo.periodic[2] && !p.forced && !p.macro && !(geo.n[0] & 1) && !(geo.stride & 1) &&
            geo.n[1] <= 65535;
