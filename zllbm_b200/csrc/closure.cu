@@ -796,7 +796,7 @@ __global__ void __launch_bounds__(kLsThreads, 3) learned_step_kernel(S* __restri
         if (!valid) continue;
         const float cn = isfinite(y) ? kCUnit * fminf(fmaxf(y, 0.f), kYMax) : fallback_c;
         F1 post[19];
-        fused_collide<Coll == kMrt, true, false>(pre, post, p, F1{18.f * cn}, (const F1*)nullptr, (F1*)nullptr);
+        fused_collide<Coll == kMrt, true, false, F1, true>(pre, post, p, F1{18.f * cn}, (const F1*)nullptr, (F1*)nullptr);
         const NodeCells<D3Q19> cell(geo, box_coord(geo, dv, i));
         if (c_node) c_node[cell(0, 0, 0)] = cn;
 #pragma unroll

@@ -52,8 +52,10 @@ __device__ __forceinline__ F1 smag_omega(F1 pi2, F1 c, float tau0) { return {sma
 // 541-592) shifts the velocity by F dt / (2 rho), j is G u, the stress gains dt (F_a u_b + F_b u_a) / 2,
 // and the term Fq_q = w [3 (c - u).F + 9 (c.u)(c.F)] splits into an even part w (9 (c.u)(c.F) - 3 u.F)
 // and an odd part 3 w (c.F) per pair.
+// Rounded: 1 / rho correctly rounded (the MRT + Smagorinsky, forced and learned collisions, which have always
+// divided so); otherwise through the fast reciprocal, two ulps.
 // mac (optional): rho, ux, uy, uz.
-template <bool Mrt, bool Les, bool Forced, class V>
+template <bool Mrt, bool Les, bool Forced, class V, bool Rounded = Forced || (Mrt && Les)>
 __device__ __forceinline__ void fused_collide(const V* d, V* out, const StepParams& p, V les_c, const V* F, V* mac) {
     static_assert(!(Mrt && Forced), "the forced MRT collision has no fused form");
     auto S = [](float s) { return splat_as<V>(s); };
@@ -87,8 +89,8 @@ __device__ __forceinline__ void fused_collide(const V* d, V* out, const StepPara
         uy = vfma(hf, F[1], jy * k);
         uz = vfma(hf, F[2], jz * k);
     } else {
-        // inv_scale / rho through the fast reciprocal (two ulps; rho is close to 1)
-        const V k = each(rho, [is](float r) { return __fdividef(is, r); });
+        const V k = Rounded ? S(is) * each(rho, [](float r) { return __frcp_rn(r); })
+                            : each(rho, [is](float r) { return __fdividef(is, r); });
         ux = jx * k;
         uy = jy * k;
         uz = jz * k;
