@@ -15,8 +15,8 @@ PROGRAM = r"""
 using namespace zl;
 
 // thread t: populations of a node with rho in about [0.8, 1.2]; counts the nodes whose ux is not the rounded
-// jx / rho
-template <bool Mrt, bool Les, bool Forced, bool Rounded>
+// jx / rho; Ask: with the rounding that the learned step asks for, else the collision's own
+template <bool Mrt, bool Les, bool Forced, bool Ask>
 __global__ void check(StepParams p, int n, unsigned* off) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
@@ -28,8 +28,13 @@ __global__ void check(StepParams p, int n, unsigned* off) {
         d[q].v = ((s >> 8) * (1.f / 16777216.f) - 0.5f) * 0.08f;
         d2[q] = splat(d[q].v);
     }
-    fused_collide<Mrt, Les, Forced, F1, Rounded>(d, out, p, F1{0.18f}, F, mac);
-    fused_collide<Mrt, Les, Forced, F2, Rounded>(d2, out2, p, splat(0.18f), Fp, mac2);
+    if constexpr (Ask) {
+        fused_collide<Mrt, Les, Forced, F1, true>(d, out, p, F1{0.18f}, F, mac);
+        fused_collide<Mrt, Les, Forced, F2, true>(d2, out2, p, splat(0.18f), Fp, mac2);
+    } else {
+        fused_collide<Mrt, Les, Forced>(d, out, p, F1{0.18f}, F, mac);
+        fused_collide<Mrt, Les, Forced>(d2, out2, p, splat(0.18f), Fp, mac2);
+    }
     const F1 X1 = (d[7] - d[10]) - (d[8] - d[9]), X2 = (d[11] - d[14]) - (d[12] - d[13]);
     const F1 jx = (d[1] - d[2]) + (X1 + X2);
     const float want = __fmul_rn(jx.v, __frcp_rn(mac[0].v));
@@ -48,9 +53,9 @@ int main() {
     p.dt = 1.;
     unsigned *off, h[8];
     if (cudaMalloc(&off, sizeof(h)) != cudaSuccess || cudaMemset(off, 0, sizeof(h)) != cudaSuccess) return 1;
-    check<true, true, false, true><<<n / 256, 256>>>(p, n, off);
+    check<true, true, false, false><<<n / 256, 256>>>(p, n, off);
     check<false, true, false, true><<<n / 256, 256>>>(p, n, off + 2);
-    check<false, true, true, true><<<n / 256, 256>>>(p, n, off + 4);
+    check<false, true, true, false><<<n / 256, 256>>>(p, n, off + 4);
     check<false, false, false, false><<<n / 256, 256>>>(p, n, off + 6);
     if (cudaMemcpy(h, off, sizeof(h), cudaMemcpyDeviceToHost) != cudaSuccess) return 1;
     for (unsigned v : h) std::printf("%u ", v);
@@ -70,8 +75,6 @@ def test_rounded_reciprocal(tmp_path):
     assert off[6] > 0  # the fast reciprocal, which the others must not be, shows in the same count
 
 
-def test_default_by_collision():
-    """Which collisions ask for it without being told to, and the learned step, which tells."""
-    csrc = os.path.join(ROOT, "zllbm_b200", "csrc")
-    assert "bool Rounded = Forced || (Mrt && Les)>" in open(os.path.join(csrc, "fused_collide.cuh")).read()
-    assert "fused_collide<Coll == kMrt, true, false, F1, true>" in open(os.path.join(csrc, "closure.cu")).read()
+def test_the_learned_step_asks():
+    src = open(os.path.join(ROOT, "zllbm_b200", "csrc", "closure.cu")).read()
+    assert "fused_collide<Coll == kMrt, true, false, F1, true>" in src

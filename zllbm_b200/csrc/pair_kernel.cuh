@@ -40,10 +40,10 @@ template <> struct PairIO<__nv_bfloat16> {
     }
 };
 
-// The unforced collision of a node pair.
-template <bool Mrt>
+// The unforced collision of a node pair in storage S.
+template <bool Mrt, class S>
 __device__ __forceinline__ void fused_pair(const F2* d, F2* out, const StepParams& p) {
-    fused_collide<Mrt, false, false>(d, out, p, splat(0.f), (const F2*)nullptr, (F2*)nullptr);
+    fused_collide<Mrt, false, false, F2, false, Mrt || sizeof(S) == 2>(d, out, p, splat(0.f), (const F2*)nullptr, (F2*)nullptr);
 }
 
 // Nodes x0 and x0 + 1 of a row of a full periodic box (or a slab of one, geo.ring: z neighbours
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(256, 2) aa_pair_kernel(S* __restrict__ f, Leve
         }
         fused_collide<Coll == kMrt, true, false>(pre, post, p, les_c, (const F2*)nullptr, (F2*)nullptr);
     } else {
-        fused_pair<Coll == kMrt>(pre, post, p);
+        fused_pair<Coll == kMrt, S>(pre, post, p);
     }
     if (sizeof(S) == 2 && p.sr_seed) {
         // stochastic rounding of the 16-bit stores, one random stream per node pair

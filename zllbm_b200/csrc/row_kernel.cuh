@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(128, 3) aa_row_kernel(S* __restrict__ f, Level
         F2 pre[19], post[19];
 #pragma unroll
         for (int q = 0; q < 19; ++q) pre[q] = IO::unpack(v[q].w[k]);
-        fused_pair<Coll == kMrt>(pre, post, p);
+        fused_pair<Coll == kMrt, S>(pre, post, p);
         if (sr) {
 #pragma unroll
             for (int q = 0; q < 19; ++q) v[q].w[k] = IO::pack_sr(post[q], rng.next());
