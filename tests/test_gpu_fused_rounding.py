@@ -11,12 +11,13 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 PROGRAM = r"""
 #include <cstdio>
+#include "closure.cuh"
 #include "pair_value.cuh"
 using namespace zl;
 
 // thread t: populations of a node with rho in about [0.8, 1.2]; counts the nodes whose ux is not the rounded
-// jx / rho; Ask: with the rounding that the learned step asks for, else the collision's own
-template <bool Mrt, bool Les, bool Forced, bool Ask>
+// jx / rho; Learned: with the reciprocal that the learned step's features leave
+template <bool Mrt, bool Les, bool Forced, bool Learned>
 __global__ void check(StepParams p, int n, unsigned* off) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
@@ -28,9 +29,13 @@ __global__ void check(StepParams p, int n, unsigned* off) {
         d[q].v = ((s >> 8) * (1.f / 16777216.f) - 0.5f) * 0.08f;
         d2[q] = splat(d[q].v);
     }
-    if constexpr (Ask) {
-        fused_collide<Mrt, Les, Forced, F1, true>(d, out, p, F1{0.18f}, F, mac);
-        fused_collide<Mrt, Les, Forced, F2, true>(d2, out2, p, splat(0.18f), Fp, mac2);
+    if constexpr (Learned) {
+        F1 x[closure::kIn], r;
+        F2 x2[closure::kIn], r2;
+        closure::fused_features(d, p, (float)p.tau, x, r);
+        closure::fused_features(d2, p, (float)p.tau, x2, r2);
+        fused_collide<Mrt, Les, Forced>(d, out, p, F1{0.18f}, F, mac, &r);
+        fused_collide<Mrt, Les, Forced>(d2, out2, p, splat(0.18f), Fp, mac2, &r2);
     } else {
         fused_collide<Mrt, Les, Forced>(d, out, p, F1{0.18f}, F, mac);
         fused_collide<Mrt, Les, Forced>(d2, out2, p, splat(0.18f), Fp, mac2);
@@ -75,6 +80,7 @@ def test_rounded_reciprocal(tmp_path):
     assert off[6] > 0  # the fast reciprocal, which the others must not be, shows in the same count
 
 
-def test_the_learned_step_asks():
+def test_the_learned_step_hands_its_reciprocal_on():
     src = open(os.path.join(ROOT, "zllbm_b200", "csrc", "closure.cu")).read()
-    assert "fused_collide<Coll == kMrt, true, false, F1, true>" in src
+    body = src[src.index("learned_step_kernel(S*"):src.index("static cudaError_t learned_step_s")]
+    assert "fused_features(pre, p, (float)p.tau, x, inv_rho)" in body and "(F1*)nullptr, &inv_rho)" in body

@@ -763,7 +763,7 @@ __global__ void __launch_bounds__(kLsThreads, 3) learned_step_kernel(S* __restri
     for (uint32_t base = blockIdx.x * kLsThreads; base < nn; base += gridDim.x * kLsThreads) {
         const uint32_t i = base + tid;
         const bool valid = i < nn;
-        F1 pre[19];
+        F1 pre[19], inv_rho;
         {
             const NodeCells<D3Q19> cell(geo, box_coord(geo, dv, valid ? i : 0u));
 #pragma unroll
@@ -774,7 +774,7 @@ __global__ void __launch_bounds__(kLsThreads, 3) learned_step_kernel(S* __restri
         }
         {
             F1 x[kIn];
-            fused_features(pre, p, (float)p.tau, x);
+            fused_features(pre, p, (float)p.tau, x, inv_rho);
             float v[32];
 #pragma unroll
             for (int j = 0; j < kIn; j += 4) {
@@ -796,7 +796,7 @@ __global__ void __launch_bounds__(kLsThreads, 3) learned_step_kernel(S* __restri
         if (!valid) continue;
         const float cn = isfinite(y) ? kCUnit * fminf(fmaxf(y, 0.f), kYMax) : fallback_c;
         F1 post[19];
-        fused_collide<Coll == kMrt, true, false, F1, true>(pre, post, p, F1{18.f * cn}, (const F1*)nullptr, (F1*)nullptr);
+        fused_collide<Coll == kMrt, true, false>(pre, post, p, F1{18.f * cn}, (const F1*)nullptr, (F1*)nullptr, &inv_rho);
         const NodeCells<D3Q19> cell(geo, box_coord(geo, dv, i));
         if (c_node) c_node[cell(0, 0, 0)] = cn;
 #pragma unroll

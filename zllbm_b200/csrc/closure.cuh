@@ -299,9 +299,9 @@ __device__ __forceinline__ void features(float rho, const float* neq, float tau0
 // The same features of a node (F1) or a node pair (F2) from its deviations d (scaled units), in the closed
 // forms of fused_collide: the relaxed moments and the stress of f - feq from the pair sums of d and the
 // equilibrium's moments, no per-direction feq.  m9 = 2 Pxx - Pyy - Pzz, m11 = Pyy - Pzz, m13..15 the off-diagonal
-// stress.
+// stress.  inv_rho: 1 / rho, correctly rounded, for the collision.
 template <class V>
-__device__ __forceinline__ void fused_features(const V* d, const StepParams& p, float tau0, V* x) {
+__device__ __forceinline__ void fused_features(const V* d, const StepParams& p, float tau0, V* x, V& inv_rho) {
     auto S = [](float s) { return splat_as<V>(s); };
     const V S1 = d[1] + d[2], D1 = d[1] - d[2];
     const V S2 = d[3] + d[4], D2 = d[3] - d[4];
@@ -321,6 +321,7 @@ __device__ __forceinline__ void fused_features(const V* d, const StepParams& p, 
     const V zero = S(0.f), is = S(p.inv_scale);
     const V rho = vfma(drho, is, S(1.f));
     const V r = each(rho, [](float v) { return __frcp_rn(v); });
+    inv_rho = r;
     const V k = is * r;  // unscaled over rho
     const V ux = (D1 + X12) * k, uy = (D2 + Y12) * k, uz = (D3 + Z12) * k;
     const V ux2 = ux * ux, uy2 = uy * uy, uz2 = uz * uz;

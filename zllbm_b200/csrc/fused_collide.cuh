@@ -52,16 +52,17 @@ __device__ __forceinline__ F1 smag_omega(F1 pi2, F1 c, float tau0) { return {sma
 // 541-592) shifts the velocity by F dt / (2 rho), j is G u, the stress gains dt (F_a u_b + F_b u_a) / 2,
 // and the term Fq_q = w [3 (c - u).F + 9 (c.u)(c.F)] splits into an even part w (9 (c.u)(c.F) - 3 u.F)
 // and an odd part 3 w (c.F) per pair.
-// Rounded: 1 / rho correctly rounded (the MRT + Smagorinsky, forced and learned collisions, which have always
-// divided so); otherwise through the fast reciprocal, two ulps.
+// 1 / rho is correctly rounded in the MRT + Smagorinsky and the forced collisions and the caller's in the learned
+// step (inv_rho, rounded too), which have always divided so; otherwise the fast reciprocal, two ulps.
 // mac (optional): rho, ux, uy, uz.
 // Planes: the two diagonal pairs of a coordinate plane share the even part that is symmetric in them, which
 // MRT corrects once for both.  An SRT pair from its own (c.u)^2 instead is as many operations in a shorter
 // chain, which the one-node kernel is bound by (us per step, 64^3 6.73 -> 6.61, between walls 256^3 546 -> 535,
 // Smagorinsky 161 x 97 x 81 36.8 -> 36.1, between walls 37.2 -> 36.5; pairs with Smagorinsky, 256^3, within
 // 0.7 %).  The 16-bit storages keep the bits of the shared form.
-template <bool Mrt, bool Les, bool Forced, class V, bool Rounded = Forced || (Mrt && Les), bool Planes = Mrt>
-__device__ __forceinline__ void fused_collide(const V* d, V* out, const StepParams& p, V les_c, const V* F, V* mac) {
+template <bool Mrt, bool Les, bool Forced, class V, bool Planes = Mrt>
+__device__ __forceinline__ void fused_collide(const V* d, V* out, const StepParams& p, V les_c, const V* F, V* mac,
+                                              const V* inv_rho = nullptr) {
     static_assert(!(Mrt && Forced), "the forced MRT collision has no fused form");
     auto S = [](float s) { return splat_as<V>(s); };
     const float* lam = p.mrt_coef;
@@ -94,8 +95,10 @@ __device__ __forceinline__ void fused_collide(const V* d, V* out, const StepPara
         uy = vfma(hf, F[1], jy * k);
         uz = vfma(hf, F[2], jz * k);
     } else {
-        const V k = Rounded ? S(is) * each(rho, [](float r) { return __frcp_rn(r); })
-                            : each(rho, [is](float r) { return __fdividef(is, r); });
+        V k;
+        if (inv_rho) k = S(is) * *inv_rho;
+        else if constexpr (Mrt && Les) k = S(is) * each(rho, [](float r) { return __frcp_rn(r); });
+        else k = each(rho, [is](float r) { return __fdividef(is, r); });
         ux = jx * k;
         uy = jy * k;
         uz = jz * k;

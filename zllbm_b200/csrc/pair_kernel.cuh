@@ -43,7 +43,7 @@ template <> struct PairIO<__nv_bfloat16> {
 // The unforced collision of a node pair in storage S.
 template <bool Mrt, class S>
 __device__ __forceinline__ void fused_pair(const F2* d, F2* out, const StepParams& p) {
-    fused_collide<Mrt, false, false, F2, false, Mrt || sizeof(S) == 2>(d, out, p, splat(0.f), (const F2*)nullptr, (F2*)nullptr);
+    fused_collide<Mrt, false, false, F2, Mrt || sizeof(S) == 2>(d, out, p, splat(0.f), (const F2*)nullptr, (F2*)nullptr);
 }
 
 // Nodes x0 and x0 + 1 of a row of a full periodic box (or a slab of one, geo.ring: z neighbours
