@@ -1,7 +1,5 @@
-// The fused D3Q19 collisions of FP32 storage and of the learned step, written once for one node (F1) and for a
-// pair of nodes in packed FP32 registers (F2 of pair_value.cuh), and those of the 16-bit pair and row kernels.
-// The 16-bit one-node kernel and forced MRT levels keep the contracted forms of aa_kernel.cuh, which their
-// results have always been rounded with.
+// The fused D3Q19 collisions of the reduced-precision storages, written once for one node (F1) and
+// for a pair of nodes in packed FP32 registers (F2 of pair_value.cuh).
 //
 // Every operation is explicit (no product and sum left for the compiler to contract), so a node's
 // result has the same bits whether a kernel updates it alone or as half of a pair, and step kernels
