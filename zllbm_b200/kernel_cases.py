@@ -83,10 +83,12 @@ def train_case(samples: int, steps: int = 3) -> float:
     g.manual_seed(7)
     x = torch.randn(samples, zl.MLP_IN, device="cuda", generator=g)
     y = torch.rand(samples, device="cuda", generator=g)
+    torch.cuda.synchronize()
+    # a stream of its own: 0, the default stream, would leave the trainer on one that the events do not see
+    stream = torch.cuda.Stream()
     with zl.Trainer(initial_net(1)) as tr:
-        tr.set_stream(torch.cuda.current_stream().cuda_stream)
-        ms = _events(torch.cuda.current_stream().cuda_stream,
-                     lambda: tr.step(x.data_ptr(), y.data_ptr(), samples, 1e-3), steps)
+        tr.set_stream(stream.cuda_stream)
+        ms = _events(stream.cuda_stream, lambda: tr.step(x.data_ptr(), y.data_ptr(), samples, 1e-3), steps)
         loss = tr.loss()
     rate = samples * steps / (ms * 1e-3) / 1e6
     print(f"train {samples} samples x {steps} steps: {rate:.1f} M samples/s, last batch loss {loss:.4g}", flush=True)
