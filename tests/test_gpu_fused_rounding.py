@@ -31,9 +31,8 @@ __global__ void check(StepParams p, int n, unsigned* off) {
     }
     if constexpr (Learned) {
         F1 x[closure::kIn], r;
-        F2 x2[closure::kIn], r2;
         closure::fused_features(d, p, (float)p.tau, x, r);
-        closure::fused_features(d2, p, (float)p.tau, x2, r2);
+        const F2 r2 = splat(r.v);
         fused_collide<Mrt, Les, Forced>(d, out, p, F1{0.18f}, F, mac, &r);
         fused_collide<Mrt, Les, Forced>(d2, out2, p, splat(0.18f), Fp, mac2, &r2);
     } else {

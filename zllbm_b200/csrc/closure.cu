@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(128) mlp_forward_kernel(const float* __restric
         for (int k = 0; k < kIn; ++k) xv[k] = valid ? x[g * kIn + k] : 0.f;
         write_x_row(it.a1s, xv, mean, istd, valid);
         float y;
-        if (!(ok = infer_tiles<1>(it, phase, err, &y))) break;
+        if (!(ok = infer_tiles<1>(it, phase, err, y))) break;
         if (valid) out[g] = y;
     }
     infer_teardown<1>(it, ok, phase);
@@ -732,15 +732,16 @@ __global__ void pairs_stage2_kernel(Grid3 g, const float* __restrict__ filt, con
 // sqrt(2 Pi:Pi)) - tau0), the Smagorinsky collision of fused_collide with C = 18 c, and streams; c is also
 // stored per node (c_node) for the steps that reuse it.
 //
-// Bound by its instructions and the waits between its phases (HBM at an eighth, tensor cores at a
-// twentieth).  The features and the collision come from the pair sums of the populations in closed form,
-// only the populations are kept across the network (the collision forms everything else again, which is
-// cheaper than registers), and the GELU leaves its factor 1/2 to the next layer's weights.  Two tiles per
+// Bound by its instructions and the waits between its phases (issue slots 63 %, HBM at a fifth of its copy
+// rate, tensor cores 7 %).  The features and the collision come from the pair sums of the populations in closed
+// form, only the populations and 1 / rho are kept across the network (the collision forms everything else again,
+// which is cheaper than registers), and the GELU leaves its factor 1/2 to the next layer's weights.  Two tiles per
 // CTA share the weights and each barrier, so that three CTAs of 80 registers (24 warps) fit an SM.  Two
 // nodes per thread as packed FP32 pairs execute a fifth fewer instructions and are slower (16 warps);
 // four CTAs of 64 registers are slower too.
-// us per step, SRT, one tile and one node per thread with per-direction equilibria / now: 33^3 69 / 12.6
-// (the weights' staging), 64^3 89 / 31, 128^3 236 / 184, 256^3 1411 / 1380.
+// us per step of one run, one tile and one node per thread with per-direction equilibria / now: SRT 33^3 69 / 12.9
+// (the weights' staging), 64^3 89 / 31.8, 128^3 238 / 187, 256^3 1409 / 1400; MRT 128^3 256 / 191, 256^3
+// 1544 / 1431.
 // The grid is the number of CTAs that fit on the GPU (shared memory 55 KiB, TMEM 128 columns per CTA).
 constexpr int kLsTiles = 2, kLsThreads = kLsTiles * kTile;
 
@@ -792,7 +793,7 @@ __global__ void __launch_bounds__(kLsThreads, 3) learned_step_kernel(S* __restri
             for (int c = 0; c < 4; ++c) st_row_chunk(tile, tid & (kTile - 1), 8 * c, kSboA1, v + 8 * c);
         }
         float y;
-        if (!(ok = infer_tiles<kLsTiles, 1>(it, phase, err, &y))) break;
+        if (!(ok = infer_tiles<kLsTiles>(it, phase, err, y))) break;
         if (!valid) continue;
         const float cn = isfinite(y) ? kCUnit * fminf(fmaxf(y, 0.f), kYMax) : fallback_c;
         F1 post[19];

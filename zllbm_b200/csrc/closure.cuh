@@ -144,8 +144,8 @@ __device__ __forceinline__ bool wait_mma(uint64_t* bar, uint32_t& phase, int* er
     return !failed;
 }
 
-// Inference of N tiles of 128 rows: X (this thread's row of each tile written by the caller) -> y of this
-// thread's rows.  64 TMEM columns per tile (Z1, then Z2).  A tile's X occupies the first 32 columns of its
+// Inference of N tiles of 128 rows: X (this thread's row written by the caller) -> y of this thread's
+// row.  64 TMEM columns per tile (Z1, then Z2).  A tile's X occupies the first 32 columns of its
 // A1 tile, whose constant columns lie beyond: X is dead once the first product is done, so the tile
 // needs no memory of its own.  Returns false if a tensor-core wait gave up.
 static_assert(tc::extent_kmajor(128, kSboA1, 2) <= kBytesA1, "X in the A1 tile as A (K = 32)");
@@ -157,10 +157,10 @@ struct InferTile {
     float b3;
 };
 
-// R rows per thread: R = N with 128 threads (a thread's rows in all tiles), R = 1 with 128 N threads.
-template <int N, int R = N>
-__device__ __forceinline__ bool infer_tiles(const InferTile& it, uint32_t& phase, int* err, float* y) {
-    const int tid = threadIdx.x, row = tid & (kTile - 1), first = R == N ? 0 : tid / kTile;
+// 128 N threads, a row each.
+template <int N>
+__device__ __forceinline__ bool infer_tiles(const InferTile& it, uint32_t& phase, int* err, float& y) {
+    const int tid = threadIdx.x, row = tid & (kTile - 1), tile = tid / kTile;
     tc::fence_proxy_async();
     tc::fence_before_sync();
     __syncthreads();
@@ -173,10 +173,10 @@ __device__ __forceinline__ bool infer_tiles(const InferTile& it, uint32_t& phase
         tc::commit(it.bar);
     }
     if (!wait_mma(it.bar, phase, err)) return false;
-    // (the loops over tiles and column halves stay loops: unrolled, the step kernel's body outgrows the
-    // instruction cache, a quarter of its stalls)
+    // (the loops over column halves stay loops: unrolled, the step kernel's body outgrows the instruction
+    // cache)
 #pragma unroll 1
-    for (int h = 2 * first; h < 2 * (first + R); ++h) {  // half h: tile h / 2, columns 32 (h % 2) ..
+    for (int h = 2 * tile; h < 2 * tile + 2; ++h) {  // half h: tile h / 2, columns 32 (h % 2) ..
         float v[32];
         tc::tmem_ld32(it.tmem + it.lane_addr + 32 * h, v);
         uint8_t* dst = it.a1s + kBytesA1 * (h >> 1) + tc::tile_offset(row, 32 * (h & 1), kSboA1);
@@ -204,7 +204,7 @@ __device__ __forceinline__ bool infer_tiles(const InferTile& it, uint32_t& phase
     if (!wait_mma(it.bar, phase, err)) return false;
     float2 acc = make_float2(it.b3, 0.f);
 #pragma unroll 1
-    for (int h = 2 * first; h < 2 * (first + R); ++h) {
+    for (int h = 2 * tile; h < 2 * tile + 2; ++h) {
         float v[32];
         tc::tmem_ld32(it.tmem + it.lane_addr + 32 * h, v);
         const float* w3 = it.w3 + 32 * (h & 1);
@@ -218,13 +218,8 @@ __device__ __forceinline__ bool infer_tiles(const InferTile& it, uint32_t& phase
             acc = __ffma2_rn(a0, make_float2(w.x, w.y), acc);
             acc = __ffma2_rn(a1, make_float2(w.z, w.w), acc);
         }
-        if (h & 1) {
-#pragma unroll
-            for (int t = 0; t < R; ++t)
-                if ((h >> 1) == first + t) y[t] = acc.x + acc.y;
-            acc = make_float2(it.b3, 0.f);
-        }
     }
+    y = acc.x + acc.y;
     return true;
 }
 
@@ -296,12 +291,12 @@ __device__ __forceinline__ void features(float rho, const float* neq, float tau0
     if (spp) *spp = s2;
 }
 
-// The same features of a node (F1) or a node pair (F2) from its deviations d (scaled units), in the closed
+// The same features of a node from its deviations d (scaled units), in the closed
 // forms of fused_collide: the relaxed moments and the stress of f - feq from the pair sums of d and the
 // equilibrium's moments, no per-direction feq.  m9 = 2 Pxx - Pyy - Pzz, m11 = Pyy - Pzz, m13..15 the off-diagonal
 // stress.  inv_rho: 1 / rho, correctly rounded, for the collision.
-template <class V>
-__device__ __forceinline__ void fused_features(const V* d, const StepParams& p, float tau0, V* x, V& inv_rho) {
+__device__ __forceinline__ void fused_features(const F1* d, const StepParams& p, float tau0, F1* x, F1& inv_rho) {
+    using V = F1;
     auto S = [](float s) { return splat_as<V>(s); };
     const V S1 = d[1] + d[2], D1 = d[1] - d[2];
     const V S2 = d[3] + d[4], D2 = d[3] - d[4];
