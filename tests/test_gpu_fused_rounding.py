@@ -82,4 +82,4 @@ def test_rounded_reciprocal(tmp_path):
 def test_the_learned_step_hands_its_reciprocal_on():
     src = open(os.path.join(ROOT, "zllbm_b200", "csrc", "closure.cu")).read()
     body = src[src.index("learned_step_kernel(S*"):src.index("static cudaError_t learned_step_s")]
-    assert "fused_features(pre, p, (float)p.tau, x, inv_rho)" in body and "(F1*)nullptr, &inv_rho)" in body
+    assert "fused_features(pre, p, (float)p.tau, x, inv_rho)" in body and "Coll == kMrt ? (const F1*)nullptr : &inv_rho)" in body

@@ -734,8 +734,8 @@ __global__ void pairs_stage2_kernel(Grid3 g, const float* __restrict__ filt, con
 //
 // Bound by its instructions and the waits between its phases (issue slots 63 %, HBM at a fifth of its copy
 // rate, tensor cores 7 %).  The features and the collision come from the pair sums of the populations in closed
-// form, only the populations and 1 / rho are kept across the network (the collision forms everything else again,
-// which is cheaper than registers), and the GELU leaves its factor 1/2 to the next layer's weights.  Two tiles per
+// form, only the populations (SRT: and 1 / rho) are kept across the network (the collision forms everything else
+// again, which is cheaper than registers), and the GELU leaves its factor 1/2 to the next layer's weights.  Two tiles per
 // CTA share the weights and each barrier, so that three CTAs of 80 registers (24 warps) fit an SM.  Two
 // nodes per thread as packed FP32 pairs execute a fifth fewer instructions and are slower (16 warps);
 // four CTAs of 64 registers are slower too.
@@ -797,7 +797,10 @@ __global__ void __launch_bounds__(kLsThreads, 3) learned_step_kernel(S* __restri
         if (!valid) continue;
         const float cn = isfinite(y) ? kCUnit * fminf(fmaxf(y, 0.f), kYMax) : fallback_c;
         F1 post[19];
-        fused_collide<Coll == kMrt, true, false>(pre, post, p, F1{18.f * cn}, (const F1*)nullptr, (F1*)nullptr, &inv_rho);
+        // (MRT forms 1 / rho again: held across the network it costs 10 steps and the read-out at 160^3, runs in
+        // turn, 3383 us against 3297; SRT the other way round, 3.17 ms against 3.21)
+        fused_collide<Coll == kMrt, true, false>(pre, post, p, F1{18.f * cn}, (const F1*)nullptr, (F1*)nullptr,
+                                                 Coll == kMrt ? (const F1*)nullptr : &inv_rho);
         const NodeCells<D3Q19> cell(geo, box_coord(geo, dv, i));
         if (c_node) c_node[cell(0, 0, 0)] = cn;
 #pragma unroll
