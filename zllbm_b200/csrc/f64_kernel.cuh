@@ -7,7 +7,7 @@
 // FP64 operations per SM and cycle the node costs 15 cycles of an SM against 14 for its 304 bytes of
 // HBM traffic: everything else has to stay out of the way.  Hence
 //  * the matrix travels in the kernel's parameters (constant bank, read through the uniform path)
-//    instead of 361 global loads per node, which kept the load pipe 77 % busy;
+//    instead of 361 global loads per node;
 //  * every row of the matrix is formed and stored at once, so that the node holds its populations and
 //    f - feq in registers and no post-collision array (no local-memory traffic);
 //  * SRT divides by the level's relaxation time through a precomputed reciprocal (DivByConstant).

@@ -1,5 +1,7 @@
-// The fused D3Q19 collisions of the reduced-precision storages, written once for one node (F1) and
-// for a pair of nodes in packed FP32 registers (F2 of pair_value.cuh).
+// The fused D3Q19 collisions of FP32 storage and of the learned step, written once for one node (F1) and for a
+// pair of nodes in packed FP32 registers (F2 of pair_value.cuh), and those of the 16-bit pair and row kernels.
+// The 16-bit one-node kernel and forced MRT levels keep the contracted forms of aa_kernel.cuh, which their
+// results have always been rounded with.
 //
 // Every operation is explicit (no product and sum left for the compiler to contract), so a node's
 // result has the same bits whether a kernel updates it alone or as half of a pair, and step kernels
@@ -52,8 +54,9 @@ __device__ __forceinline__ F1 smag_omega(F1 pi2, F1 c, float tau0) { return {sma
 // 541-592) shifts the velocity by F dt / (2 rho), j is G u, the stress gains dt (F_a u_b + F_b u_a) / 2,
 // and the term Fq_q = w [3 (c - u).F + 9 (c.u)(c.F)] splits into an even part w (9 (c.u)(c.F) - 3 u.F)
 // and an odd part 3 w (c.F) per pair.
-// 1 / rho is correctly rounded in the MRT + Smagorinsky and the forced collisions and the caller's in the learned
-// step (inv_rho, rounded too), which have always divided so; otherwise the fast reciprocal, two ulps.
+// 1 / rho is correctly rounded in the MRT + Smagorinsky and the forced collisions and the caller's where it has
+// it (inv_rho: the learned SRT step, rounded too), which have always divided so; otherwise the fast reciprocal,
+// two ulps.
 // mac (optional): rho, ux, uy, uz.
 // Planes: the two diagonal pairs of a coordinate plane share the even part that is symmetric in them, which
 // MRT corrects once for both.  An SRT pair from its own (c.u)^2 instead is as many operations in a shorter
