@@ -29,19 +29,26 @@ int main() {
     auto expect = [&](bool a, bool b) { bad += a != b; };
     for (int n : {128, 256}) {
         for (const auto* p : {&les, &plain}) {
-            expect(zl::pair_default(3, *p, 4, level(n, n, n, 0)), true);
-            for (int block : {32, 64, 128, 256}) expect(zl::pair_default(3, *p, 4, level(n, n, n, block)), false);
-            expect(zl::pair_default(3, *p, 4, level(n - 1, n, n, 0)), false);
-            expect(zl::pair_default(3, *p, 4, level(32, 32, 32, 0)), false);
-            expect(zl::pair_default(3, *p, 2, level(n, n, n, 0)), false);
-            expect(zl::pair_default(3, *p, 8, level(n, n, n, 0)), false);
+            expect(zl::pair_default(3, false, *p, 4, level(n, n, n, 0)), true);
+            for (int block : {32, 64, 128, 256}) expect(zl::pair_default(3, false, *p, 4, level(n, n, n, block)), false);
+            expect(zl::pair_default(3, false, *p, 4, level(n - 1, n, n, 0)), false);
+            expect(zl::pair_default(3, false, *p, 4, level(32, 32, 32, 0)), false);
+            expect(zl::pair_default(3, false, *p, 2, level(n, n, n, 0)), false);
+            expect(zl::pair_default(3, false, *p, 8, level(n, n, n, 0)), false);
         }
         for (int block : {-64, 0, 64}) expect(zl::pair_les_eligible(3, les, 4, level(n, n, n, block)), true);
     }
-    // rows that leave lanes idle: 33 of 64 and 45 of 64 never, 23 of 32 and 75 of 96 with Smagorinsky only
-    for (int n : {66, 90}) expect(zl::pair_default(3, les, 4, level(n, 200, 200, 0)), false);
-    for (int n : {46, 150}) expect(zl::pair_default(3, les, 4, level(n, 200, 200, 0)), true);
-    for (int n : {46, 66, 90, 150}) expect(zl::pair_default(3, plain, 4, level(n, 200, 200, 0)), false);
+    // rows that leave lanes idle: 33 of 64 and 45 of 64 never, 23 of 32 and 75 of 96 with Smagorinsky only, and 23
+    // of 32 on smaller levels with MRT only
+    for (bool mrt : {false, true}) {
+        expect(zl::pair_default(3, mrt, les, 4, level(46, 150, 150, 0)), mrt);
+        expect(zl::pair_default(3, mrt, les, 4, level(46, 200, 200, 0)), true);
+        expect(zl::pair_default(3, mrt, les, 4, level(96, 96, 96, 0)), true);
+        expect(zl::pair_default(3, mrt, les, 4, level(66, 200, 200, 0)), false);
+    }
+    for (int n : {66, 90}) expect(zl::pair_default(3, false, les, 4, level(n, 200, 200, 0)), false);
+    for (int n : {46, 150}) expect(zl::pair_default(3, false, les, 4, level(n, 200, 200, 0)), true);
+    for (int n : {46, 66, 90, 150}) expect(zl::pair_default(3, false, plain, 4, level(n, 200, 200, 0)), false);
     expect(zl::pair_les_eligible(3, plain, 4, level(128, 128, 128, -64)), false);
     expect(zl::pair_les_eligible(3, les, 4, level(129, 128, 128, -64)), false);
     expect(zl::pair_les_eligible(3, les, 2, level(128, 128, 128, -64)), false);

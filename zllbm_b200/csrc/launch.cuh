@@ -84,17 +84,18 @@ inline bool pair_les_eligible(int dims, const StepParams& p, int elem_bytes, con
 // are numbered for.
 // Measured us per step, one node / two nodes per thread:
 //                   80^3          96^3          112^3         128^3         256^3
-//   SRT          11.3 / 13.3   16.4 / 18.0   36.3 / 37.5   54.2 / 52.8   403 / 384
-//   MRT          12.3 / 14.3   19.5 / 19.0   40.0 / 39.0   58.4 / 53.6   435 / 385
-//   SRT + LES    14.4 / 15.5   22.9 / 20.7   47.0 / 40.0   67.7 / 53.7   508 / 389
-//   MRT + LES    18.9 / 18.1   30.6 / 24.1   55.0 / 42.2   77.9 / 55.6   581 / 407
+//   SRT          10.6 / 12.9   15.8 / 17.5   35.3 / 37.4   53.6 / 53.3   407 / 385
+//   MRT          12.3 / 14.6   18.7 / 19.2   38.8 / 39.2   56.6 / 53.6   448 / 398
+//   SRT + LES    13.6 / 16.1   21.7 / 21.4   45.8 / 40.7   66.2 / 54.3   508 / 405
+//   MRT + LES    16.8 / 18.1   28.8 / 24.0   52.8 / 42.5   75.1 / 56.0   581 / 424
 // and only where the row's pairs fill enough of the lanes launched for them: nine tenths (150^3, 75 pairs on 96
-// lanes: SRT 87 / 92, MRT 94 / 98), with Smagorinsky, whose one-node kernel is bound by its instructions, five
-// sevenths (one / two nodes per thread, SRT + LES and MRT + LES; share of the lanes in front):
-//   .52  66 x 161 x 150  52.5 / 59.3   59.2 / 63.4       .72  46 x 150 x 150   27.1 / 26.1   34.7 / 29.2
-//   .63  80 x 90 x 90    16.6 / 18.6   20.1 / 21.1       .77  98 x 90 x 90     20.4 / 19.9   24.8 / 21.9
-//   .68  130 x 70 x 70   17.4 / 19.8   20.8 / 21.5       .78  150 x 100 x 100  49.4 / 46.3   55.6 / 48.0
-//   .70  90 x 90 x 90    19.3 / 19.5   23.2 / 21.6       .94  60 x 150 x 150   43.1 / 37.7   50.2 / 38.9
+// lanes: SRT 86 / 96, MRT 92 / 100); with Smagorinsky, whose one-node kernel is bound by its instructions, five
+// sevenths, and three quarters for SRT below kPairMinNodes (SRT + LES, MRT + LES; share of the lanes in front):
+//   .52  66 x 161 x 150  51.4 / 60.4   60.3 / 64.0       .72  46 x 150 x 150   26.2 / 27.4   34.7 / 29.8
+//   .63  80 x 90 x 90    16.2 / 18.9   20.7 / 21.5       .72  46 x 200 x 200   60.7 / 57.5   68.6 / 60.2
+//   .68  130 x 70 x 70   16.9 / 19.9   21.0 / 21.9       .77  98 x 90 x 90     19.9 / 20.2   25.0 / 22.3
+//   .70  90 x 90 x 90    18.8 / 19.8   23.4 / 22.0       .78  150 x 100 x 100  48.8 / 46.3   56.0 / 48.5
+//   .71  136 x 100 x 120 53.4 / 53.2   60.8 / 55.9       .94  60 x 150 x 150   43.1 / 37.8   50.5 / 39.4
 constexpr long long kPairMinNodes = 3ll << 19, kPairMinNodesLes = 1ll << 19;
 // Threads along x of the pair kernel's default blocks: the widest rows that leave the fewest lanes idle.
 inline int pair_lanes(int n0, int bx) { return (n0 / 2 + bx - 1) / bx * bx; }
@@ -104,11 +105,13 @@ inline int pair_block_x(int n0) {
         if (pair_lanes(n0, w) < pair_lanes(n0, bx)) bx = w;
     return bx;
 }
-inline bool pair_default(int dims, const StepParams& p, int elem_bytes, const LevelGeom& geo) {
+inline bool pair_default(int dims, bool mrt, const StepParams& p, int elem_bytes, const LevelGeom& geo) {
     const long long nodes = (long long)geo.n[0] * geo.n[1] * geo.n[2];
     if (geo.block[0] != 0 || nodes < (p.les ? kPairMinNodesLes : kPairMinNodes)) return false;
     const int pairs = geo.n[0] / 2, lanes = pair_lanes(geo.n[0], pair_block_x(geo.n[0]));
-    if (p.les) return 7 * pairs >= 5 * lanes && pair_les_eligible(dims, p, elem_bytes, geo);
+    if (p.les)
+        return (mrt || nodes >= kPairMinNodes ? 7 * pairs >= 5 * lanes : 4 * pairs >= 3 * lanes) &&
+               pair_les_eligible(dims, p, elem_bytes, geo);
     return 10 * pairs >= 9 * lanes && dims == 3 && elem_bytes == 4 && geo.full && geo.periodic[0] &&
            geo.periodic[1] && geo.periodic[2] && !p.forced && !p.macro && !(geo.n[0] & 1) && !(geo.stride & 1) &&
            geo.n[1] <= 65535;

@@ -110,7 +110,7 @@ cudaError_t step_lco(bool bnd, bool masked, S* f, const LevelGeom& geo, const St
         if (geo.block[0] < 0 && pair_eligible(3, bnd, masked, p, (int)sizeof(S), geo))
             return step_pair<S, C, O, false>(f, geo, p, s);
         if constexpr (sizeof(S) == 4) {
-            if (pair_default(3, p, (int)sizeof(S), geo) ||
+            if (pair_default(3, C == kMrt, p, (int)sizeof(S), geo) ||
                 (geo.block[0] < 0 && pair_les_eligible(3, p, (int)sizeof(S), geo)))
                 return p.les ? step_pair<S, C, O, true>(f, geo, p, s) : step_pair<S, C, O, false>(f, geo, p, s);
         }
