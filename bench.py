@@ -371,7 +371,7 @@ def run_ours(args):
     if args.tune:
         ctx.set_populations(0, codes, f0)
     ctx.set_graph(args.graph)
-    # the graph is captured by the first zl_advance of two or more steps, inside the warm-up
+    # (a step of one launch on this many nodes gains nothing from a graph and is launched directly)
     if args.graph:
         ctx.advance(args.warmup)
     else:

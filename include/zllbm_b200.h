@@ -225,10 +225,10 @@ int zl_set_level_streams(zl_ctx* ctx, int enabled);
 
 /* Replay zl_advance as captured CUDA graphs of an even number of background steps (every launch
    of the sub-cycled order, transfers and boundary passes included): pairs of steps, and for a
-   single level up to sixteen once a few hundred steps have been asked for; steps that are one
-   launch each and fill no such graph, and the last of an odd number, are launched directly.  The
-   graphs are re-captured after any change of levels, interfaces, vertices or tuning.  Off by
-   default. */
+   single level up to sixteen once some steps have been asked for.  Where a step is one launch,
+   those that fill no such graph are launched directly, and all of them on levels of more than
+   four million nodes; so is the last of an odd number.  The graphs are re-captured after any
+   change of levels, interfaces, vertices or tuning.  Off by default. */
 int zl_set_graph(zl_ctx* ctx, int enabled);
 
 /* Thread-block shape of a level's step kernel: x (a multiple of 32) by y threads, at most 256;

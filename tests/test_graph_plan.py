@@ -12,14 +12,15 @@ PROGRAM = r"""
 #include <cstdio>
 #include <cstdlib>
 #include "graph_plan.h"
-// arguments: single_level one_launch calls...; prints per call: run runs pairs direct captured
+// arguments: single_level one_launch nodes calls...; prints per call: run runs pairs direct captured
 int main(int argc, char** argv) {
     const bool single = std::atoi(argv[1]), one = std::atoi(argv[2]);
+    const long long nodes = std::atoll(argv[3]);
     long long seen = 0;
     int have = 0;
-    for (int i = 3; i < argc; ++i) {
+    for (int i = 4; i < argc; ++i) {
         const int steps = std::atoi(argv[i]);
-        const zl::GraphPlan p = zl::plan_graph(steps, single, one, seen, have);
+        const zl::GraphPlan p = zl::plan_graph(steps, single, one, nodes, seen, have);
         seen += steps;
         const bool captured = p.runs > 0 && p.run != have;
         if (p.runs > 0) have = p.run;
@@ -36,8 +37,8 @@ def plan(tmp_path_factory):
     subprocess.run(["g++", "-std=c++17", "-I", os.path.join(ROOT, "zllbm_b200", "csrc"), str(d / "plan.cpp"), "-o",
                     str(d / "plan")], check=True)
 
-    def run(single, one, calls):
-        out = subprocess.run([str(d / "plan"), str(int(single)), str(int(one)), *map(str, calls)], capture_output=True,
+    def run(single, one, calls, nodes=30000):
+        out = subprocess.run([str(d / "plan"), str(int(single)), str(int(one)), str(nodes), *map(str, calls)], capture_output=True,
                              text=True, check=True).stdout
         rows = [tuple(map(int, line.split())) for line in out.splitlines()]
         for steps, (length, runs, pairs, direct, captured) in zip(calls, rows):
@@ -69,3 +70,9 @@ def test_a_program_of_short_calls_gets_a_graph_of_their_length(plan):
 
 def test_multi_level_steps_replay_in_pairs(plan):
     assert plan(False, False, [3, 300, 2]) == [(0, 0, 1, 1, 0), (0, 0, 150, 0, 0), (0, 0, 1, 0, 0)]
+
+
+def test_long_steps_of_one_launch_take_no_graph(plan):
+    assert plan(True, True, [1000, 3], 1 << 24) == [(0, 0, 0, 1000, 0), (0, 0, 0, 3, 0)]
+    assert plan(True, True, [1000], 1 << 22)[0][:2] == (16, 62)
+    assert plan(True, False, [1000], 1 << 24)[0][:2] == (16, 62)

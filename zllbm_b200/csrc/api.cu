@@ -1189,7 +1189,8 @@ int zl_advance(zl_ctx* ctx, int steps) {
     }
     const bool single_level = ctx->cfg.max_level == 0;
     const bool one_launch = single_level && !ctx->levels[0].ordered && ctx->levels[0].n_vertices == 0;
-    const GraphPlan plan = plan_graph(steps, single_level, one_launch, ctx->graph_steps_seen, valid(run) ? run.steps : 0);
+    const GraphPlan plan = plan_graph(steps, single_level, one_launch, ctx->levels[0].nodes, ctx->graph_steps_seen,
+                                      valid(run) ? run.steps : 0);
     ctx->graph_steps_seen += steps;
     int rc;
     if (plan.runs > 0 && !(valid(run) && run.steps == plan.run) &&

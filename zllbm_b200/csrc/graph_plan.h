@@ -19,8 +19,13 @@ namespace zl {
 // a few dozen steps and is read out must not pay that, so a single level's long graph is captured once
 // kLongGraphAfter steps have been asked for.  First call of 8 / 40 steps: 33^2 175 / 316 us with the long graph
 // at once, 52 / 196 now; the ordered 33 x 25 x 21 464 / 1419 and 308 / 1081.
+// Above kGraphMaxNodes a step of one launch outlasts the next one's launch and gains nothing from a graph
+// (launched / in graphs of 16: 192^3 FP32 176 / 177, FP16 177.6 / 177.4, FP64 553 / 552; 256^3 FP32 398 / 399, FP64
+// 1184 / 1184; below it the channel of 161 x 97 x 81 still gains 0.7 %), while instantiating one asks the driver
+// for memory: a timed call that did so beside a starting nvidia-smi took 87 ms longer.  Such steps are always
+// launched directly.
 constexpr int kGraphSteps = 16, kGraphMinSteps = 8;
-constexpr long long kLongGraphAfter = 128;
+constexpr long long kLongGraphAfter = 128, kGraphMaxNodes = 1ll << 22;
 
 struct GraphPlan {
     int run = 0;     // steps of the level's long graph (more than it holds now: capture it), 0: none
@@ -31,9 +36,9 @@ struct GraphPlan {
 
 // seen: steps that earlier calls asked for since the last change of the set-up; have: steps that the
 // long graph holds, 0 if there is none.  A multi-level step is dozens of launches and replays in pairs.
-inline GraphPlan plan_graph(int steps, bool single_level, bool one_launch, long long seen, int have) {
+inline GraphPlan plan_graph(int steps, bool single_level, bool one_launch, long long nodes, long long seen, int have) {
     GraphPlan p;
-    if (single_level) {
+    if (single_level && !(one_launch && nodes > kGraphMaxNodes)) {
         const int most = std::min(kGraphSteps, steps & ~1);
         p.run = seen + steps >= kLongGraphAfter && most >= kGraphMinSteps ? std::max(have, most) : have;
     }
